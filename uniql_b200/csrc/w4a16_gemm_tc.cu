@@ -87,6 +87,14 @@ struct TcParams {
 
 __device__ __forceinline__ uint32_t tc_smem_addr(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
 
+// One lane of a converged warp.  The branch on elect.sync is what lets the compiler keep tcgen05 descriptors in uniform
+// registers: under a plain `lane == 0` branch every tcgen05.mma carries a per-lane loop around its operands, 48 cycles
+// an instruction however small N is, against 10 (N = 16), 32 (N = 64) and 128 (N = 256) here.
+__device__ __forceinline__ bool tc_elect() {
+  uint32_t e;
+  asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(e));
+  return e != 0;
+}
 __device__ __forceinline__ void tc_mbar_init(uint32_t bar, uint32_t count) {
   asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count) : "memory");
 }
@@ -305,7 +313,7 @@ w4a16_gemm_tc_kernel(const TcParams p, const __grid_constant__ CUtensorMap amap)
 
   if (warp == 0) {
     // ------------------------------------------------------------------ activation producer
-    if (lane == 0) {
+    if (tc_elect()) {
       int it_ab = 0;
       for (int tile = blockIdx.x; tile < total_tiles; tile += gridDim.x) {
         const int mt = tile % p.mtiles;
@@ -321,7 +329,7 @@ w4a16_gemm_tc_kernel(const TcParams p, const __grid_constant__ CUtensorMap amap)
     }
   } else if (warp == 1) {
     // ------------------------------------------------------------------ MMA issuer
-    if (lane == 0) {
+    if (tc_elect()) {
       int it_ab = 0, it_tile = 0;
       uint32_t ready = 0;                        // the current stage's full barrier was seen complete by the last poll
       for (int tile = blockIdx.x; tile < total_tiles; tile += gridDim.x, ++it_tile) {
@@ -674,7 +682,7 @@ w4a16_gemm_tc_swap_kernel(const __grid_constant__ TcSwapParams p, const __grid_c
 
   if (warp == 0) {
     // ------------------------------------------------------------------ packed-weight producer (the HBM stream)
-    if (lane == 0) {
+    if (tc_elect()) {
       int it = 0;
       for (int nt = tile0; nt < p.ntiles; nt += tile_step) {
         int pi, lt;
@@ -689,7 +697,7 @@ w4a16_gemm_tc_swap_kernel(const __grid_constant__ TcSwapParams p, const __grid_c
     }
   } else if (warp == 2) {
     // ------------------------------------------------------------------ activation producer (re-reads, L2 hits)
-    if (lane == 0) {
+    if (tc_elect()) {
       // Programmatic dependent launch: everything up to here (barriers, tensor memory, the first weight tiles, the
       // dequantise warps' scale loads) ran while the producer of the activations was still finishing; the activation
       // tiles are the only thing that has to wait for it.  Results are stored after MMAs that consumed those tiles.
@@ -706,7 +714,7 @@ w4a16_gemm_tc_swap_kernel(const __grid_constant__ TcSwapParams p, const __grid_c
     }
   } else if (warp == 1) {
     // ------------------------------------------------------------------ MMA issuer
-    if (lane == 0) {
+    if (tc_elect()) {
       int it = 0, it_tile = 0;
       uint32_t ready = 0;                        // the current stage's full barrier was seen complete by the last poll
       for (int nt = tile0; nt < p.ntiles; nt += tile_step, ++it_tile) {
@@ -870,7 +878,7 @@ w4a16_gemm_tc_swap_kernel(const __grid_constant__ TcSwapParams p, const __grid_c
       asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
       tc_fence_before();
       __syncwarp();
-      if (lane == 0) {
+      if (tc_elect()) {
         tc_mbar_arrive(bar_full + 8 * s);
         tc_mbar_arrive(bar_empty_p + 8 * sp);
       }
