@@ -320,6 +320,11 @@ int uniql_w4a16_plan_selftest(int64_t m, int64_t k, const int64_t* n, int nproj,
  * that failed; out5 (may be NULL) receives {WN, S, cluster (0/1), dynamic shared memory bytes, partial-sum bytes}. */
 int uniql_w4a16_gemv_plan_check(int64_t m, int64_t k, const int64_t* n, int nproj, int epilogue, int64_t* out5);
 
+/* Host-only check of every plan the operand-swapped tensor-core kernel can be launched with (ring depths against the
+ * number of dequantise sets and issuing threads, tensor-memory columns, shared memory).  Returns 0, or the row-tile size
+ * whose plan breaks a rule the kernel relies on. */
+int uniql_w4a16_swap_plan_check(void);
+
 #ifdef __cplusplus
 }
 #endif

@@ -109,3 +109,10 @@ def test_tiled_kernel_plan_check_refuses_bad_shapes(built_lib):
     assert _tiled_plan(1, 4000, [4096])[0] == 1           # k must be a multiple of 128
     assert _tiled_plan(1, 4096, [4096, 2048], 1)[0] == 2  # SwiGLU needs two equal widths
     assert _tiled_plan(1, 4096, [100])[0] == 3            # widths are multiples of 64
+
+
+def test_swap_kernel_plans(built_lib):
+    """Ring depths, tensor memory and shared memory of every row tile of the operand-swapped kernel: a packed ring that is
+    no multiple of the dequantise sets, or a stage ring shorter than them, lets a wait pass on an older phase."""
+    from uniql_b200._lib import lib
+    assert lib().uniql_w4a16_swap_plan_check() == 0

@@ -79,8 +79,10 @@ static int group_launch(const CommView* cv, int64_t k_offset, const void* A, int
       ds[i] = proj[i].D;
       widths[i] = proj[i].n;
     }
-    if (!gemm_tc_group_supported(m, k, widths, nproj)) return UNIQL_ESHAPE;
-    return launch_gemm_tc_group(la, ds, nproj, (const __half*)A, lda, m, stream);
+    if (!gemm_swap_supported(m, k, widths, nproj)) return UNIQL_ESHAPE;
+    SwapArgs sa{};
+    sa.projs = la; sa.Ds = ds; sa.nproj = nproj; sa.A = (const __half*)A; sa.lda = lda; sa.m = m;
+    return launch_gemm_swap(sa, stream);
   }
   if (epilogue != UNIQL_EPILOGUE_NONE && epilogue != UNIQL_EPILOGUE_SWIGLU) return UNIQL_EINVAL;
   if (epilogue == UNIQL_EPILOGUE_SWIGLU && (nproj != 2 || proj[0].n != proj[1].n || proj[0].n_out != proj[1].n_out))

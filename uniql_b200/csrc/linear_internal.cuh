@@ -80,11 +80,20 @@ struct LinearArgs {
 bool gemm_tc_supported(int64_t m, int64_t n, int64_t k);
 size_t gemm_tc_scratch_bytes(int64_t m, int64_t n, int64_t k);
 int launch_gemm_tc(const LinearArgs& a, const __half* A, int64_t lda, __half* D, int64_t m, cudaStream_t stream);
-// 16 < m <= 128: up to kMaxProj projections that read the same activations (same k) as one launch of the
-// operand-swapped kernel; Ds[i] receives projection i (leading dimension projs[i].ldd).
-bool gemm_tc_group_supported(int64_t m, int64_t k, const int64_t* n, int nproj);
-int launch_gemm_tc_group(const LinearArgs* projs, void* const* Ds, int nproj, const __half* A, int64_t lda, int64_t m,
-                         cudaStream_t stream);
+// Operand-swapped tensor-core kernel (w4a16_gemm_swap.cu): up to kMaxProj projections that read the same activations
+// (same k) as one launch; Ds[i] receives projection i (leading dimension projs[i].ldd).
+struct SwapArgs {
+  const LinearArgs* projs;
+  void* const* Ds;
+  int nproj;
+  bool pair;                  // projections 0 and 1 are gate and up: Ds[0] receives silu(gate) * up
+  const void* residual;       // fp16 [m, n_out] added to the rounded result, or nullptr
+  int64_t ldr;
+  const __half* A;
+  int64_t lda, m;
+};
+bool gemm_swap_supported(int64_t m, int64_t k, const int64_t* n, int nproj);
+int launch_gemm_swap(const SwapArgs& a, cudaStream_t stream);
 
 // Hadamard transform of fp16 rows (used by the fused linear); signals dependents early when pdl is set.
 int launch_hadamard(const void* x, int64_t ldx, void* y, int64_t ldy, int64_t rows, int64_t dim, float scale,

@@ -1083,6 +1083,8 @@ static int launch_variant(const DecodeParams& p, const DecodePlan& pl, cudaStrea
   return UNIQL_OK;
 }
 
+constexpr int kSwapMinRows = 5;
+
 int launch_decode(const DecodeArgs& a, cudaStream_t stream) {
   int64_t n[kMaxProj] = {0, 0, 0, 0};
   if (a.nproj < 1 || a.nproj > kMaxProj) return UNIQL_EINVAL;
@@ -1112,6 +1114,24 @@ int launch_decode(const DecodeArgs& a, cudaStream_t stream) {
       }
       if (st != UNIQL_OK) return st;
       lda = a.hadamard_dim;
+    }
+    // From five rows on the tensor-core kernel with exact codes as the operand and fp32 group scales (the arithmetic of the
+    // tiled kernel) is faster: its work per weight does not grow with the rows, while the tiled kernel stages rows x k
+    // activations in every CTA.  14336 x 4096 in us, tiled / tensor core: 4 rows 9.8 / 11.4, 8 rows 12.8 / 11.7, 16 rows
+    // 18.6 / 11.7; 4096 x 14336: 11.8 / 12.6, 13.9 / 12.7, 18.7 / 12.8; 4096 x 4096: 6.7 / 7.6, 7.1 / 7.5, 8.5 / 7.6.
+    if (!a.comm && a.m >= kSwapMinRows && gemm_swap_supported(a.m, a.k, n, a.nproj)) {
+      LinearArgs la[kMaxProj];
+      void* ds[kMaxProj];
+      for (int i = 0; i < a.nproj; ++i) {
+        const DecodeProjArgs& q = a.proj[i];
+        la[i].B = q.B; la[i].s = q.s; la[i].bias = q.bias; la[i].ldd = q.ldd;
+        la[i].n = q.n; la[i].n_out = q.n_out; la[i].k = a.k; la[i].status_word = a.status_word;
+        ds[i] = q.D;
+      }
+      SwapArgs sa{};
+      sa.projs = la; sa.Ds = ds; sa.nproj = a.nproj; sa.pair = a.epilogue == UNIQL_EPILOGUE_SWIGLU;
+      sa.residual = a.residual; sa.ldr = a.ldr; sa.A = Ain; sa.lda = lda; sa.m = a.m;
+      return launch_gemm_swap(sa, stream);
     }
     return launch_gemv_group(a, Ain, lda, stream);
   }
