@@ -37,6 +37,19 @@ def test_rows_and_widths(m, n, k):
         _check(ops.w4a16_linear(x.cuda(), w, s, b, n), x, layer)
 
 
+@pytest.mark.parametrize("n,k", [(128, 128), (192, 640), (4096, 1024), (9600, 256)])
+@pytest.mark.parametrize("m", [129, 209, 225, 256, 257, 301, 600])
+def test_more_than_128_rows(m, n, k):
+    """Row tiles of 144 to 256 rows (four, three and two stages), several row tiles, split over k, and the 256 x 256 tiles
+    of the prefill kernel where they are chosen."""
+    from uniql_b200 import ops
+    layer = quantized_layer(n + k, n, k, bias=(n == 192))
+    x = make_acts(m, m, k)
+    w, s, b, _ = _dev(layer)
+    for _ in range(2):
+        _check(ops.w4a16_linear(x.cuda(), w, s, b, n), x, layer)
+
+
 @pytest.mark.parametrize("m", [7, 16, 18, 64, 128])
 @pytest.mark.parametrize("widths,k", [((192, 128, 448), 384), ((9600, 9664), 256)])
 def test_groups(m, widths, k):

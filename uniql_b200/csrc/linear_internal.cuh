@@ -94,6 +94,7 @@ struct SwapArgs {
 };
 bool gemm_swap_supported(int64_t m, int64_t k, const int64_t* n, int nproj);
 int launch_gemm_swap(const SwapArgs& a, cudaStream_t stream);
+double gemm_swap_cycles(int64_t m, int64_t k, int ctiles);   // modelled SM cycles of such a launch
 
 // Hadamard transform of fp16 rows (used by the fused linear); signals dependents early when pdl is set.
 int launch_hadamard(const void* x, int64_t ldx, void* y, int64_t ldy, int64_t rows, int64_t dim, float scale,

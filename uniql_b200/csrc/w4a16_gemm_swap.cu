@@ -53,6 +53,7 @@ constexpr int FIRST_EPI_WARP = 4, FIRST_DEQ_WARP = 8;
 constexpr int THREADS = (FIRST_DEQ_WARP + NSETS * DEQ_WARPS) * 32;
 constexpr int FINISH_THREADS = THREADS - FIRST_EPI_WARP * 32;
 constexpr int NUM_BARS = 3 * MAX_STAGES + 2 * MAX_PSTAGES + 4;
+constexpr int MB_MAX = 256;                     // rows of a tile
 constexpr int RC = 16;                          // batch rows per epilogue chunk
 constexpr int ROW_BYTES = BNW * 4;              // one batch row of a parked fp32 tile
 constexpr int OFF_BAR = 0, OFF_PART = 1024, OFF_P = OFF_PART + 2 * RC * ROW_BYTES;
@@ -778,11 +779,57 @@ static SwapPlan swap_plan(int Mb, bool gs, bool one_tile, int min_kb) {
 static bool swap_plan_ok(const SwapPlan& pl, int Mb, bool gs) {
   using namespace sw;
   const int acc_cols = gs ? pl.nst * 16 : pl.nbuf * pl.nissue * Mb;
-  return Mb >= 16 && Mb <= 256 && Mb % 16 == 0 && pl.nst >= 2 && pl.nst <= MAX_STAGES && pl.nsets >= 1 && pl.nsets <= NSETS &&
+  return Mb >= 16 && Mb <= MB_MAX && Mb % 16 == 0 && pl.nst >= 2 && pl.nst <= MAX_STAGES && pl.nsets >= 1 && pl.nsets <= NSETS &&
          pl.nst >= pl.nsets && pl.nst % pl.nissue == 0 && pl.pst >= pl.nsets && pl.pst <= MAX_PSTAGES && pl.pst % pl.nsets == 0 &&
          acc_cols + pl.nst * (BK / 2) <= TMEM_COLS && pl.off_x % 1024 == 0 && pl.off_x >= OFF_P + pl.pst * P_BYTES &&
          pl.off_x + pl.nst * Mb * BK * 2 + 1024 <= pl.smem && pl.smem <= SMEM_MAX &&
          Mb * ROW_BYTES <= pl.nst * Mb * BK * 2;
+}
+
+// Row tiles and k-split of a launch: the cheapest of a few by a model of its cycles.  A stage (128 columns x Mb rows x
+// 128 k) takes 4 Mb cycles of the tensor pipe, but no less than ~430 of the dequantise warps; a wave of tiles whose
+// epilogue has no second accumulator to hide behind adds ~20 cycles a row; a cluster sum ~3000.  14336 x 4096, 160 rows:
+// 628 cycles a stage measured (640 by the pipe), 224 rows 865 (896); above 224 rows the activation ring has room for two
+// stages only: 256 rows 1153 (1024).
+struct SwapShape {
+  int rtiles, Mb, split;
+  double cycles;
+};
+static SwapShape swap_shape(int64_t m, int64_t k, int ctiles, bool gs) {
+  using namespace sw;
+  static const int forced = swap_env("UNIQL_B200_TC_SPLIT", 0);
+  const int sms = device_info().sm_count;
+  const int groups = (int)(k / 128);
+  SwapShape best{};
+  best.cycles = 1e30;
+  const int rt0 = (int)((m + MB_MAX - 1) / MB_MAX), rt1 = m <= 128 ? 1 : rt0 + 2;
+  for (int rt = rt0; rt <= rt1; ++rt) {
+    const int Mb = (int)(((m + rt - 1) / rt + 15) / 16 * 16);
+    if ((int64_t)(rt - 1) * Mb >= m) continue;
+    const int64_t tiles = (int64_t)ctiles * rt;
+    const double stage = Mb > 224 ? 4.5 * Mb : Mb > 107 ? 4.0 * Mb : 430.0;
+    for (int split = 1; split <= 8; ++split) {
+      if (forced > 0 ? split != (forced > groups ? groups : forced) : (split > 1 && (tiles * split > sms || groups / split < 4)))
+        continue;
+      // every cluster must be resident at once (a second wave would cost more than the split gains): clusters are placed
+      // inside one GPC, so fewer fit than SMs / split suggests
+      if (split > 1 && forced <= 0 &&
+          swap_max_clusters(gs, split, swap_plan(Mb, gs, true, groups / split).smem) < tiles)
+        continue;
+      const int64_t waves = split > 1 ? 1 : (tiles + sms - 1) / sms;
+      const double epi = (Mb > 128 || waves == 1) ? 20.0 * Mb : 0.0;
+      const double cycles = waves * (((groups + split - 1) / split) * stage + epi) + (split > 1 ? 3000.0 : 0.0);
+      if (cycles < best.cycles) { best.cycles = cycles; best.rtiles = rt; best.Mb = Mb; best.split = split; }
+    }
+  }
+  return best;
+}
+
+// The model's figure for a launch of `ctiles` 128-column tiles (the kernel's attributes must have been set: see there).
+static int swap_set_attributes(bool gs, bool pair);
+double gemm_swap_cycles(int64_t m, int64_t k, int ctiles) {
+  if (swap_set_attributes(m <= 16, false) != UNIQL_OK) return 1e30;
+  return swap_shape(m, k, ctiles, m <= 16).cycles;
 }
 
 bool gemm_swap_supported(int64_t m, int64_t k, const int64_t* n, int nproj) {
@@ -790,6 +837,21 @@ bool gemm_swap_supported(int64_t m, int64_t k, const int64_t* n, int nproj) {
   for (int i = 0; i < nproj; ++i)
     if (n[i] < 128 || n[i] % 64) return false;
   return true;
+}
+
+// Function attributes are per device; the occupancy query behind the k-split needs them too (always on the plain kernel).
+static int swap_set_attributes(bool gs, bool pair) {
+  static thread_local bool set[64][4] = {};
+  int dev = 0;
+  cudaGetDevice(&dev);
+  if (dev < 0 || dev >= 64) dev = 0;
+  for (int pr = 0; pr <= (pair ? 1 : 0); ++pr) {
+    bool& done = set[dev][(gs ? 2 : 0) + pr];
+    if (done) continue;
+    UNIQL_CUDA_TRY(cudaFuncSetAttribute(swap_kernel(gs, pr != 0), cudaFuncAttributeMaxDynamicSharedMemorySize, sw::SMEM_MAX));
+    done = true;
+  }
+  return UNIQL_OK;
 }
 
 int launch_gemm_swap(const SwapArgs& a, cudaStream_t stream) {
@@ -802,8 +864,6 @@ int launch_gemm_swap(const SwapArgs& a, cudaStream_t stream) {
   memset(&p, 0, sizeof(p));
   SwapMaps wmaps;
   p.pair = a.pair ? 1 : 0;
-  p.rtiles = (int)((m + 255) / 256);
-  const int Mb = (int)(((m + p.rtiles - 1) / p.rtiles + 15) / 16 * 16);
   int ctiles = 0;
   for (int i = 0; i < a.nproj; ++i) {
     const LinearArgs& q = a.projs[i];
@@ -821,7 +881,15 @@ int launch_gemm_swap(const SwapArgs& a, cudaStream_t stream) {
   for (int i = a.nproj; i < kMaxProj; ++i) { wmaps.w[i] = wmaps.w[0]; p.proj[i] = p.proj[0]; }
   p.nproj = a.nproj;
   p.residual = (const __half*)a.residual; p.ldr = a.ldr;
+  const bool gs = m <= 16;
+  {
+    const int st = swap_set_attributes(gs, a.pair);
+    if (st != UNIQL_OK) return st;
+  }
+  const SwapShape shape = swap_shape(m, k, ctiles, gs);
+  const int Mb = shape.Mb, split = shape.split, sms = device_info().sm_count;
   p.M = (int)m; p.Mb = Mb; p.K = (int)k;
+  p.rtiles = shape.rtiles;
   p.ntiles = ctiles * p.rtiles;
   p.status_word = a.projs[0].status_word;
   CUtensorMap xmap;
@@ -835,42 +903,6 @@ int launch_gemm_swap(const SwapArgs& a, cudaStream_t stream) {
             CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
             CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
       return cuda_fail(cudaErrorInvalidValue);
-  }
-  const bool gs = m <= 16;
-  {
-    // function attributes are per device
-    static thread_local bool attr_set[64][4] = {};
-    int dev = 0;
-    cudaGetDevice(&dev);
-    if (dev < 0 || dev >= 64) dev = 0;
-    const int which = (gs ? 2 : 0) + (a.pair ? 1 : 0);
-    if (!attr_set[dev][which]) {
-      UNIQL_CUDA_TRY(cudaFuncSetAttribute(swap_kernel(gs, a.pair), cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_MAX));
-      if (a.pair) UNIQL_CUDA_TRY(cudaFuncSetAttribute(swap_kernel(gs, false), cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_MAX));
-      attr_set[dev][which] = true;
-    }
-  }
-  const int sms = device_info().sm_count;
-  // few tiles: a cluster of `split` CTAs shares each tile, every CTA reducing a slice of k (at least four scale groups)
-  int split = 1;
-  {
-    static const int forced = swap_env("UNIQL_B200_TC_SPLIT", 0);
-    const int groups = (int)(k / 128);
-    if (forced > 0) split = forced;
-    else if (p.ntiles * 2 <= sms) {
-      split = sms / p.ntiles;
-      if (split > 8) split = 8;
-      while (split > 1 && groups / split < 4) --split;
-    }
-    if (split > groups) split = groups;
-    if (split < 1) split = 1;
-    if (split > 8) split = 8;
-    if (split > 1) {
-      // every cluster must be resident at once (a second wave would cost more than the split gains): clusters are
-      // placed inside one GPC, so fewer fit than SMs / split suggests
-      const int smem = swap_plan(Mb, gs, true, groups / split).smem;
-      while (split > 1 && forced <= 0 && swap_max_clusters(gs, split, smem) < p.ntiles) --split;
-    }
   }
   p.split = split;
   p.one_tile = split > 1 || p.ntiles <= sms;
@@ -909,7 +941,7 @@ int launch_gemm_swap(const SwapArgs& a, cudaStream_t stream) {
 // Host-only check (no device work): every row tile this kernel can be launched with gets a plan that its barriers, tensor
 // memory and shared memory can hold.  0, or the row-tile size whose plan fails.
 extern "C" int uniql_w4a16_swap_plan_check(void) {
-  for (int Mb = 16; Mb <= 256; Mb += 16)
+  for (int Mb = 16; Mb <= uniql::sw::MB_MAX; Mb += 16)
     for (int one = 0; one < 2; ++one)
       for (int gs = 0; gs <= (Mb == 16 ? 1 : 0); ++gs)
         for (int kb = 1; kb <= 2; ++kb)

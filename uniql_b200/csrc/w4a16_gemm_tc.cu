@@ -1,24 +1,21 @@
-// Prefill-regime W4A16 linear (m > 16) for sm_100a: tcgen05 tensor cores with the accumulator in TMEM and the
-// int4 -> fp16 dequantisation done on the SM in front of the MMA.  Two kernels:
-//   w4a16_gemm_tc_kernel<H>      m > 128: activations are the 128-row operand, dequantised weights the N operand
-//                                (shared memory);
-//   w4a16_gemm_tc_swap_kernel    16 < m <= 128: operands swapped, dequantised weights written to tensor memory.
+// Prefill-regime W4A16 linear for sm_100a: tcgen05 tensor cores with the accumulator in TMEM and the int4 -> fp16
+// dequantisation done on the SM in front of the MMA, on 256 x 256 tiles.  Also the dispatch between this kernel and the
+// operand-swapped one (w4a16_gemm_swap.cu) for more than 16 rows.
 //
 // Replaces the large-batch instantiations of UniQL's Marlin kernel (csrc/linear/marlin_gemm_kernel.cuh:176-740,
 // tile table :802-810), which run mma.sync with dequantisation on the same warps, while consuming the same
 // packed buffers (quantize/quantize_helpers.py:145-165 weight order, :54-62 scale order).
 //
-// w4a16_gemm_tc_kernel<H>.  Tile: (128 * H) batch rows x 256 output columns x 64 k per pipeline stage, one persistent
-// CTA per SM.  H = 2 when the 256-row tiles still fill the GPU: the two 128-row halves are separate M=128 MMAs that
-// read the same dequantised weight tile, which halves the dequantisation work and the shared-memory writes per
-// tensor-core cycle; their accumulators are the two 256-column halves of TMEM.  H = 1 double-buffers one accumulator
-// across tiles instead.
+// w4a16_gemm_tc_kernel.  Tile: 256 batch rows x 256 output columns x 64 k per pipeline stage, one persistent CTA per SM.
+// The two 128-row halves are separate M=128 MMAs that read the same dequantised weight tile, which halves the
+// dequantisation work and the shared-memory writes per tensor-core cycle; their accumulators are the two 256-column
+// halves of TMEM.
 //   warp 0      TMA producer: activation tile(s) [128 x 64] fp16 (128B-swizzled, K-major); no multicast.
 //   warp 1      allocates TMEM (2 x 256 fp32 columns); one elected lane issues, per stage, one block of
 //               tcgen05.mma kind::f16 (M=128, N=256, K=16) + the commit that releases the stage + a poll of the next
 //               stage's barrier whose latency hides behind the MMA issue.
-//   warps 2..   epilogue (4 per 128-row half): tcgen05.ld (32 lanes x 32 columns), + bias, fp32 -> fp16, row-major
-//               stores; with H = 1 it overlaps the next tile's main loop through the second TMEM accumulator.
+//   warps 2..9  epilogue (4 per 128-row half): tcgen05.ld (32 lanes x 32 columns), + bias, fp32 -> fp16, row-major
+//               stores.
 //   16 warps    dequantise, as two sets of eight that convert alternate stages so two stages are always in
 //               conversion: packed words straight from global memory into registers (requested two stages ahead,
 //               no hop through shared memory), exact (q - 8) in fp16 via LOP3 + HSUB2/HFMA2, one HMUL2 by the group
@@ -46,19 +43,18 @@ constexpr int DEQ_SETS = 2;                   // dequantise warp sets; set t con
 constexpr int DEQ_SET_WARPS = 8;              // per set: 4 column blocks x 2 pairs of packed rows
 constexpr int DEQ_WARPS = DEQ_SETS * DEQ_SET_WARPS;
 constexpr int TMEM_COLS = 512;
-template <int H> struct Cfg {
-  static constexpr int AB_STAGES = H == 1 ? 4 : 3;
-  static constexpr int STAGE_A = H * A_BYTES;
-  static constexpr int OFF_A = 0;
-  static constexpr int OFF_B = OFF_A + AB_STAGES * STAGE_A;
-  static constexpr int OFF_BAR = OFF_B + AB_STAGES * B_BYTES;
-  static constexpr int NUM_BARS = 2 * AB_STAGES + 4;
-  static constexpr int SMEM_BYTES = OFF_BAR + NUM_BARS * 8 + 16 + 1024;   // + slack to align the base to 1 KB
-  static constexpr int FIRST_EPI_WARP = 2;
-  static constexpr int EPI_WARPS = 4 * H;
-  static constexpr int FIRST_DEQ_WARP = FIRST_EPI_WARP + EPI_WARPS;
-  static constexpr int THREADS = (FIRST_DEQ_WARP + DEQ_WARPS) * 32;
-};
+constexpr int H = 2;                          // 128-row halves of a tile
+constexpr int AB_STAGES = 3;
+constexpr int STAGE_A = H * A_BYTES;
+constexpr int OFF_A = 0;
+constexpr int OFF_B = OFF_A + AB_STAGES * STAGE_A;
+constexpr int OFF_BAR = OFF_B + AB_STAGES * B_BYTES;
+constexpr int NUM_BARS = 2 * AB_STAGES + 4;
+constexpr int SMEM_BYTES = OFF_BAR + NUM_BARS * 8 + 16 + 1024;   // + slack to align the base to 1 KB
+constexpr int FIRST_EPI_WARP = 2;
+constexpr int EPI_WARPS = 4 * H;
+constexpr int FIRST_DEQ_WARP = FIRST_EPI_WARP + EPI_WARPS;
+constexpr int THREADS = (FIRST_DEQ_WARP + DEQ_WARPS) * 32;
 // instruction descriptor: D fp32, A/B fp16, both K-major, N = 256, M = 128
 constexpr uint32_t IDESC = (1u << 4) | ((uint32_t)(BN >> 3) << 17) | ((uint32_t)(BMH >> 4) << 24);
 }  // namespace tc
@@ -78,65 +74,39 @@ struct TcParams {
 // of the NEXT stage's barrier, in one block: the poll is issued first and its result read last, so its latency hides
 // behind the issue of the MMAs instead of adding to the single issuing thread's serial time per stage.  Returns
 // whether the next stage was already full.
-template <int H>
 __device__ __forceinline__ uint32_t tc_issue_stage(uint32_t tmem_d, uint64_t adesc0, uint64_t adesc1, uint64_t bdesc,
                                                    uint32_t accumulate, uint32_t bar_release, uint32_t bar_next,
                                                    uint32_t par_next) {
   uint32_t ok;
-  if (H == 1) {
-    asm volatile(
-        "{\n\t.reg .pred p, q, t;\n\t.reg .b64 a1, a2, a3, b1, b2, b3;\n\t"
-        "mbarrier.test_wait.parity.shared::cta.b64 q, [%7], %8;\n\t"
-        "setp.ne.b32 p, %5, 0;\n\t"
-        "setp.eq.b32 t, 0, 0;\n\t"
-        "add.u64 a1, %2, 2;\n\tadd.u64 a2, %2, 4;\n\tadd.u64 a3, %2, 6;\n\t"
-        "add.u64 b1, %3, 2;\n\tadd.u64 b2, %3, 4;\n\tadd.u64 b3, %3, 6;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%1], %2, %3, %4, p;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%1], a1, b1, %4, t;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%1], a2, b2, %4, t;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%1], a3, b3, %4, t;\n\t"
-        "tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%6];\n\t"
-        "selp.u32 %0, 1, 0, q;\n\t}"
-        : "=r"(ok)
-        : "r"(tmem_d), "l"(adesc0), "l"(bdesc), "r"(tc::IDESC), "r"(accumulate), "r"(bar_release), "r"(bar_next),
-          "r"(par_next)
-        : "memory");
-  } else {
-    asm volatile(
-        "{\n\t.reg .pred p, q, t;\n\t.reg .b64 a1, a2, a3, c1, c2, c3, b1, b2, b3;\n\t.reg .b32 d1;\n\t"
-        "mbarrier.test_wait.parity.shared::cta.b64 q, [%8], %9;\n\t"
-        "setp.ne.b32 p, %6, 0;\n\t"
-        "setp.eq.b32 t, 0, 0;\n\t"
-        "add.u32 d1, %1, 256;\n\t"
-        "add.u64 a1, %2, 2;\n\tadd.u64 a2, %2, 4;\n\tadd.u64 a3, %2, 6;\n\t"
-        "add.u64 c1, %3, 2;\n\tadd.u64 c2, %3, 4;\n\tadd.u64 c3, %3, 6;\n\t"
-        "add.u64 b1, %4, 2;\n\tadd.u64 b2, %4, 4;\n\tadd.u64 b3, %4, 6;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%1], %2, %4, %5, p;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%1], a1, b1, %5, t;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%1], a2, b2, %5, t;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%1], a3, b3, %5, t;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [d1], %3, %4, %5, p;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [d1], c1, b1, %5, t;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [d1], c2, b2, %5, t;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [d1], c3, b3, %5, t;\n\t"
-        "tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%7];\n\t"
-        "selp.u32 %0, 1, 0, q;\n\t}"
-        : "=r"(ok)
-        : "r"(tmem_d), "l"(adesc0), "l"(adesc1), "l"(bdesc), "r"(tc::IDESC), "r"(accumulate), "r"(bar_release),
-          "r"(bar_next), "r"(par_next)
-        : "memory");
-  }
+  asm volatile(
+      "{\n\t.reg .pred p, q, t;\n\t.reg .b64 a1, a2, a3, c1, c2, c3, b1, b2, b3;\n\t.reg .b32 d1;\n\t"
+      "mbarrier.test_wait.parity.shared::cta.b64 q, [%8], %9;\n\t"
+      "setp.ne.b32 p, %6, 0;\n\t"
+      "setp.eq.b32 t, 0, 0;\n\t"
+      "add.u32 d1, %1, 256;\n\t"
+      "add.u64 a1, %2, 2;\n\tadd.u64 a2, %2, 4;\n\tadd.u64 a3, %2, 6;\n\t"
+      "add.u64 c1, %3, 2;\n\tadd.u64 c2, %3, 4;\n\tadd.u64 c3, %3, 6;\n\t"
+      "add.u64 b1, %4, 2;\n\tadd.u64 b2, %4, 4;\n\tadd.u64 b3, %4, 6;\n\t"
+      "tcgen05.mma.cta_group::1.kind::f16 [%1], %2, %4, %5, p;\n\t"
+      "tcgen05.mma.cta_group::1.kind::f16 [%1], a1, b1, %5, t;\n\t"
+      "tcgen05.mma.cta_group::1.kind::f16 [%1], a2, b2, %5, t;\n\t"
+      "tcgen05.mma.cta_group::1.kind::f16 [%1], a3, b3, %5, t;\n\t"
+      "tcgen05.mma.cta_group::1.kind::f16 [d1], %3, %4, %5, p;\n\t"
+      "tcgen05.mma.cta_group::1.kind::f16 [d1], c1, b1, %5, t;\n\t"
+      "tcgen05.mma.cta_group::1.kind::f16 [d1], c2, b2, %5, t;\n\t"
+      "tcgen05.mma.cta_group::1.kind::f16 [d1], c3, b3, %5, t;\n\t"
+      "tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%7];\n\t"
+      "selp.u32 %0, 1, 0, q;\n\t}"
+      : "=r"(ok)
+      : "r"(tmem_d), "l"(adesc0), "l"(adesc1), "l"(bdesc), "r"(tc::IDESC), "r"(accumulate), "r"(bar_release),
+        "r"(bar_next), "r"(par_next)
+      : "memory");
   return ok;
 }
 
-template <int H>
-__global__ void __launch_bounds__(tc::Cfg<H>::THREADS, 1)
+__global__ void __launch_bounds__(tc::THREADS, 1)
 w4a16_gemm_tc_kernel(const TcParams p, const __grid_constant__ CUtensorMap amap) {
   using namespace tc;
-  constexpr int AB_STAGES = Cfg<H>::AB_STAGES, STAGE_A = Cfg<H>::STAGE_A;
-  constexpr int OFF_A = Cfg<H>::OFF_A, OFF_B = Cfg<H>::OFF_B, OFF_BAR = Cfg<H>::OFF_BAR;
-  constexpr int NUM_BARS = Cfg<H>::NUM_BARS, FIRST_EPI_WARP = Cfg<H>::FIRST_EPI_WARP;
-  constexpr int FIRST_DEQ_WARP = Cfg<H>::FIRST_DEQ_WARP;
   static_assert(BN == 256, "the second accumulator sits 256 tensor-memory columns after the first");
   extern __shared__ uint8_t smem_unaligned[];
   // 1 KB alignment: the 128B-swizzled tiles must start on a swizzle-atom boundary
@@ -202,13 +172,10 @@ w4a16_gemm_tc_kernel(const TcParams p, const __grid_constant__ CUtensorMap amap)
       int it_ab = 0, it_tile = 0;
       uint32_t ready = 0;                        // the current stage's full barrier was seen complete by the last poll
       for (int tile = blockIdx.x; tile < total_tiles; tile += gridDim.x, ++it_tile) {
-        // H == 1: one accumulator per tile, alternating between the two TMEM halves (epilogue of tile t overlaps
-        // the main loop of tile t+1).  H == 2: both halves belong to this tile.
-        const int buf0 = H == 1 ? (it_tile & 1) : 0;
-        const uint32_t empty_parity = (H == 1 ? ((it_tile >> 1) & 1) : (it_tile & 1)) ^ 1;
+        const uint32_t empty_parity = (it_tile & 1) ^ 1;
 #pragma unroll
         for (int h = 0; h < H; ++h)
-          if (!timed_out && !tc_mbar_wait(bar_tmem_empty + 8 * (buf0 + h), empty_parity)) timed_out = true;
+          if (!timed_out && !tc_mbar_wait(bar_tmem_empty + 8 * h, empty_parity)) timed_out = true;
         tc_fence_after();
         for (int kb = 0; kb < KB; ++kb, ++it_ab) {
           const int s = it_ab % AB_STAGES;
@@ -216,25 +183,25 @@ w4a16_gemm_tc_kernel(const TcParams p, const __grid_constant__ CUtensorMap amap)
           tc_fence_after();
           const int s1 = (s + 1 == AB_STAGES) ? 0 : s + 1;
           const uint64_t adesc0 = tc_smem_desc(sbase + OFF_A + s * STAGE_A);
-          ready = tc_issue_stage<H>(tmem_base + buf0 * BN, adesc0, adesc0 + (A_BYTES >> 4),
+          ready = tc_issue_stage(tmem_base, adesc0, adesc0 + (A_BYTES >> 4),
                                     tc_smem_desc(sbase + OFF_B + s * B_BYTES), kb != 0 ? 1u : 0u, bar_empty_ab + 8 * s,
                                     bar_full + 8 * s1, ((it_ab + 1) / AB_STAGES) & 1);
           if (it_ab + 1 >= total_it) ready = 0;   // that poll looked at a phase nobody will complete
         }
 #pragma unroll
-        for (int h = 0; h < H; ++h) tc_commit(bar_tmem_full + 8 * (buf0 + h));   // accumulators complete
+        for (int h = 0; h < H; ++h) tc_commit(bar_tmem_full + 8 * h);   // accumulators complete
       }
     }
   } else if (warp < FIRST_DEQ_WARP) {
     // ------------------------------------------------------------------ epilogue
     const int q = warp & 3;                     // TMEM lane quadrant this warp may access
-    const int half = (warp - FIRST_EPI_WARP) >> 2;   // which 128-row half of the tile (always 0 when H == 1)
+    const int half = (warp - FIRST_EPI_WARP) >> 2;   // which 128-row half of the tile 
     int it_tile = 0;
     const bool vec_ok = ((p.ldd & 7) == 0) && ((reinterpret_cast<uintptr_t>(p.D) & 15u) == 0);
     for (int tile = blockIdx.x; tile < total_tiles; tile += gridDim.x, ++it_tile) {
       const int mt = tile % p.mtiles, nt = tile / p.mtiles;
-      const int buf = H == 1 ? (it_tile & 1) : half;
-      const uint32_t full_parity = H == 1 ? ((it_tile >> 1) & 1) : (it_tile & 1);
+      const int buf = half;
+      const uint32_t full_parity = it_tile & 1;
       if (!timed_out && !tc_mbar_wait_relaxed(bar_tmem_full + 8 * buf, full_parity)) timed_out = true;
       tc_fence_after();
       const int m = (mt * H + half) * BMH + q * 32 + lane;
@@ -385,9 +352,25 @@ bool gemm_tc_supported(int64_t m, int64_t n, int64_t k) {
 
 size_t gemm_tc_scratch_bytes(int64_t, int64_t, int64_t) { return 0; }
 
+// Which kernel runs m > 16 rows.  The 256 x 256 tiles of the kernel above reuse activations and weights twice as often as
+// the 128-column tiles of the operand-swapped kernel, whose finer tiles, k-split and shared launches waste less of the
+// last wave: the modelled cycles decide (a 64-k stage of a tile ~1200 cycles and ~4000 for its epilogue, against the
+// other kernel's model times the 1.12 it falls short of it by).  Measured, tiles / swapped, us: 14336 x 4096 at 301 rows
+// 72 (its 128-row form, since removed) / 38, 1024 rows 98 / 115, 4096 rows 363 / 421; 4096 x 14336 at 1024 rows
+// 120 / 95, 4096 rows 346 / 384.
+static bool prefill_tiles_win(int64_t m, int64_t n, int64_t k) {
+  static const int forced = [] { const char* e = getenv("UNIQL_B200_TC_SWAP"); return (e && *e) ? atoi(e) : -1; }();
+  if (forced >= 0) return forced == 0;
+  if (m <= 128) return false;
+  const int sms = device_info().sm_count;
+  const int64_t tiles = ((m + 255) / 256) * ((n + 255) / 256);
+  const double cycles = (double)((tiles + sms - 1) / sms) * (k / 64 * 1200.0 + 4000.0);
+  return cycles < 1.12 * gemm_swap_cycles(m, k, (int)((n + 127) / 128));
+}
+
 int launch_gemm_tc(const LinearArgs& a, const __half* A, int64_t lda, __half* D, int64_t m, cudaStream_t stream) {
   using namespace tc;
-  if (m <= 128) {
+  if (!prefill_tiles_win(m, a.n, a.k)) {
     void* d1[1] = {D};
     SwapArgs sa{};
     sa.projs = &a; sa.Ds = d1; sa.nproj = 1; sa.A = A; sa.lda = lda; sa.m = m;
@@ -409,10 +392,7 @@ int launch_gemm_tc(const LinearArgs& a, const __half* A, int64_t lda, __half* D,
   TcParams p;
   p.B = (const uint4*)a.B; p.S = (const uint4*)a.s; p.bias = (const __half*)a.bias; p.D = D; p.ldd = a.ldd;
   p.M = (int)m; p.N = (int)a.n; p.n_out = (int)a.n_out; p.K = (int)a.k;
-  // 256-row tiles share each dequantised weight tile between two MMAs; use them once they still fill the GPU
   p.ntiles = (int)((a.n + BN - 1) / BN);
-  const int sms_ = device_info().sm_count;
-  const int H = (m > BMH && ((m + 2 * BMH - 1) / (2 * BMH)) * (int64_t)p.ntiles >= sms_) ? 2 : 1;
   p.mtiles = (int)((m + H * BMH - 1) / (H * BMH));
   p.status_word = a.status_word;
   {
@@ -421,20 +401,14 @@ int launch_gemm_tc(const LinearArgs& a, const __half* A, int64_t lda, __half* D,
     cudaGetDevice(&dev);
     if (dev < 0 || dev >= 64) dev = 0;
     if (!attr_set[dev]) {
-      UNIQL_CUDA_TRY(cudaFuncSetAttribute(w4a16_gemm_tc_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                          Cfg<1>::SMEM_BYTES));
-      UNIQL_CUDA_TRY(cudaFuncSetAttribute(w4a16_gemm_tc_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                          Cfg<2>::SMEM_BYTES));
+      UNIQL_CUDA_TRY(cudaFuncSetAttribute(w4a16_gemm_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES));
       attr_set[dev] = true;
     }
   }
   const int64_t tiles = (int64_t)p.mtiles * p.ntiles;
   const int sms = device_info().sm_count;
   const int grid = (int)(tiles < sms ? tiles : sms);
-  if (H == 1)
-    w4a16_gemm_tc_kernel<1><<<grid, Cfg<1>::THREADS, Cfg<1>::SMEM_BYTES, stream>>>(p, amap);
-  else
-    w4a16_gemm_tc_kernel<2><<<grid, Cfg<2>::THREADS, Cfg<2>::SMEM_BYTES, stream>>>(p, amap);
+  w4a16_gemm_tc_kernel<<<grid, THREADS, SMEM_BYTES, stream>>>(p, amap);
   return launch_status();
 }
 
