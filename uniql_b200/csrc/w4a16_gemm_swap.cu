@@ -916,9 +916,10 @@ int launch_gemm_swap(const SwapArgs& a, cudaStream_t stream) {
   cfg.stream = stream;
   cudaLaunchAttribute attr[2];
   int nattr = 0;
-  // may start behind its predecessor; the kernel waits (griddepcontrol.wait) before it reads the activations
+  // May start behind its predecessor; the kernel waits (griddepcontrol.wait) before it reads the activations, but not for
+  // the weights and scales: callers of the entry points above 128 rows may have written those just before.
   static const int pdl_on = swap_env("UNIQL_B200_PDL", 1);
-  if (pdl_on) {
+  if (pdl_on && m <= 128) {
     attr[nattr].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[nattr].val.programmaticStreamSerializationAllowed = 1;
     ++nattr;
