@@ -124,3 +124,21 @@ def test_full_size_gate_projection_properties():
     y = ops.w4a16_linear(x, packed, scales, None, n)
     y_ref = x.float() @ w_ref.float()
     assert float((y.float() - y_ref).abs().max() / y_ref.abs().max()) <= 1e-2    # the linear path's tolerance
+
+
+@pytest.mark.parametrize("n_out,k_in", [(64, 128), (4096, 128), (1000, 333)])
+def test_rtn_without_reference_weights_on_any_bit_pattern(n_out, k_in):
+    """The kernel without reference weights against the one with them (which the oracle pins), bit for bit: every fp16 bit
+    pattern may occur -- quotients on and beside the midpoints of fp16, subnormal scales, infinities, NaN."""
+    g = torch.Generator().manual_seed(n_out + k_in)
+    bits = torch.randint(0, 1 << 16, (n_out, k_in), generator=g)
+    # most columns stay below a magnitude of their own, so that quotients fill the whole range of codes
+    cap = torch.randint(1, 0x7c00, (n_out, 1), generator=g)
+    low = (bits & 0x8000) | ((bits & 0x7fff) % (cap + 1))
+    bits = torch.where(torch.arange(n_out).reshape(-1, 1) % 4 == 0, bits, low)
+    w = torch.where(bits >= 1 << 15, bits - (1 << 16), bits).to(torch.int16).view(torch.float16).cuda()
+    from uniql_b200 import ops
+    _, packed, scales = ops.w4a16_quantize(w, want_ref=True)
+    _, packed2, scales2 = ops.w4a16_quantize(w, want_ref=False)
+    assert torch.equal(packed, packed2)
+    assert torch.equal(scales.view(torch.int16), scales2.view(torch.int16))

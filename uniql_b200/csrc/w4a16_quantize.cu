@@ -150,6 +150,106 @@ w4a16_quantize_kernel(const QuantParams p) {
   }
 }
 
+// RTN without reference weights (from_fp16 on a GPU, the re-quantisation of the slicers): nothing but the weight crosses
+// memory and nothing crosses shared memory.  A warp owns columns w and w + 8 of every 16 (lanes 0-15 / 16-31, 8
+// consecutive k each), the two columns of one packed word, so a word is put together with three shuffles.
+// What bound the kernel above here was its instructions (a division, two conversions and two byte accesses to shared
+// memory per weight: 78 us for 14336 x 4096, of which the traffic needs 23).  The quotient is taken as w * (1 / s), both
+// correctly rounded, so the exact quotient lies within two ulps; fp16 rounding can only come out differently where a
+// midpoint between two fp16 numbers lies in that interval (the low 13 bits of the product within 2 of 0x1000), and
+// those few are divided.  Rounding to an integer and the offset 8 are one fp16 addition of 1544 (ulp 1, ties to even).
+__global__ void __launch_bounds__(kQThreads)
+w4a16_quantize_rtn_kernel(const QuantParams p) {
+  const int t = threadIdx.x, w = t >> 5, lane = t & 31, h = lane >> 4, seg = lane & 15;
+  const int n0 = blockIdx.x * kTileN, k0 = blockIdx.y * kTileK;
+  const bool vec_ok = ((p.ldw & 7) == 0) && ((reinterpret_cast<uintptr_t>(p.W) & 15u) == 0);
+  uint4 raw[4];
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    const int gn = n0 + 16 * j + w + 8 * h, gk = k0 + seg * 8;
+    raw[j] = make_uint4(0, 0, 0, 0);            // rows / k past the matrix read as zero
+    if (gn < p.n_out) {
+      const __half* src = p.W + (size_t)gn * p.ldw + gk;
+      if (vec_ok && gk + 8 <= p.k_in) {
+        raw[j] = ld_nc16(src);
+      } else {
+        uint32_t v[4];
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          const uint32_t lo = gk + 2 * e < p.k_in ? __half_as_ushort(src[2 * e]) : 0u;
+          const uint32_t hi = gk + 2 * e + 1 < p.k_in ? __half_as_ushort(src[2 * e + 1]) : 0u;
+          v[e] = lo | (hi << 16);
+        }
+        raw[j] = make_uint4(v[0], v[1], v[2], v[3]);
+      }
+    }
+  }
+  // absmax per column; two columns share a half2 through the butterfly (fp16 maxima are exact)
+  __half amax[4];
+#pragma unroll
+  for (int jp = 0; jp < 2; ++jp) {
+    __half m2[2];
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+      const __half2* v = reinterpret_cast<const __half2*>(&raw[2 * jp + i]);
+      __half2 m = __float2half2_rn(0.f);
+#pragma unroll
+      for (int e = 0; e < 4; ++e) m = __hmax2(m, __habs2(v[e]));
+      m2[i] = __hmax(__low2half(m), __high2half(m));
+    }
+    __half2 both = __halves2half2(m2[0], m2[1]);
+#pragma unroll
+    for (int d = 1; d < 16; d <<= 1) both = __hmax2(both, __shfl_xor_sync(0xffffffffu, both, d));
+    amax[2 * jp] = __low2half(both);
+    amax[2 * jp + 1] = __high2half(both);
+  }
+  uint32_t words[4];
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    // fp16 tensor times the Python scalar 2/15: one fp32 multiply, one rounding to fp16
+    const __half s16 = __float2half_rn(__fmul_rn(__half2float(amax[j]), (float)(2.0 / 15.0)));
+    // stored[8 i + j'] = natural[i + 8 j'] inside the block: column 16 j + w + 8 h sits at 8 w + 2 j + h
+    if (seg == 0) p.scales[(size_t)blockIdx.y * p.n_pad + n0 + 8 * w + 2 * j + h] = s16;
+    const float s = __half2float(s16);
+    const float inv = __frcp_rn(s);
+    const __half2* v = reinterpret_cast<const __half2*>(&raw[j]);
+    uint32_t c[4], nearest = 0xffffffffu;
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      const float2 f = __half22float2(v[e]);
+      const float a = __fmul_rn(f.x, inv), b = __fmul_rn(f.y, inv);
+      nearest = min(nearest, min((__float_as_uint(a) - 0xffeu) & 0x1fffu, (__float_as_uint(b) - 0xffeu) & 0x1fffu));
+      // max first: a NaN (0 / 0, inf / inf) becomes -8, code 0
+      __half2 q = __hmin2(__hmax2(__floats2half2_rn(a, b), __float2half2_rn(-8.f)), __float2half2_rn(7.f));
+      q = __hadd2(q, __float2half2_rn(1544.f));
+      c[e] = *reinterpret_cast<const uint32_t*>(&q) & 0x000f000fu;
+    }
+    if (nearest <= 4u) {                        // a product lies within two ulps of an fp16 midpoint: divide
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        const float2 f = __half22float2(v[e]);
+        __half2 q = __floats2half2_rn(__fdiv_rn(f.x, s), __fdiv_rn(f.y, s));
+        q = __hadd2(__hmin2(__hmax2(q, __float2half2_rn(-8.f)), __float2half2_rn(7.f)), __float2half2_rn(1544.f));
+        c[e] = *reinterpret_cast<const uint32_t*>(&q) & 0x000f000fu;
+      }
+    }
+    // an all-zero group (and a padded column) has code 0; nibble (2c + 8 (seg & 1) + {0, 1}, column half h) of word c
+    const int sh = 4 * (seg & 1) + 8 * h;
+#pragma unroll
+    for (int e = 0; e < 4; ++e) c[e] = s == 0.f ? 0u : c[e] << sh;
+    // the four lanes {seg pair} x {h} hold a quarter of words 0..3 each: every lane ends up with word (seg & 1) + 2 h
+    const bool odd = seg & 1;
+    uint32_t w0 = odd ? c[1] : c[0], w1 = odd ? c[3] : c[2];
+    w0 |= __shfl_xor_sync(0xffffffffu, odd ? c[0] : c[1], 1);
+    w1 |= __shfl_xor_sync(0xffffffffu, odd ? c[2] : c[3], 1);
+    const uint32_t other = __shfl_xor_sync(0xffffffffu, h ? w0 : w1, 16);
+    words[j] = (h ? w1 : w0) | other;
+  }
+  const int kt = seg >> 1, cw = (seg & 1) + 2 * h;
+  *reinterpret_cast<uint4*>(p.packed + ((size_t)blockIdx.y * 8 + kt) * (2 * (size_t)p.n_pad) + (size_t)blockIdx.x * 128 +
+                            (w * 4 + cw) * 4) = make_uint4(words[0], words[1], words[2], words[3]);
+}
+
 }  // namespace
 
 }  // namespace uniql
@@ -173,7 +273,8 @@ extern "C" int uniql_w4a16_quantize(const void* W, int64_t ldw, int64_t n_out, i
   if (groups > 65535) return UNIQL_ESHAPE;
   dim3 grid((unsigned)(n_pad / 64), (unsigned)groups);
   cudaStream_t stream = (cudaStream_t)stream_;
-  if (group_scale) w4a16_quantize_kernel<true><<<grid, kQThreads, 0, stream>>>(p);
+  if (!group_scale && !w_ref && aligned16(packed)) w4a16_quantize_rtn_kernel<<<grid, kQThreads, 0, stream>>>(p);
+  else if (group_scale) w4a16_quantize_kernel<true><<<grid, kQThreads, 0, stream>>>(p);
   else w4a16_quantize_kernel<false><<<grid, kQThreads, 0, stream>>>(p);
   return launch_status();
 }
