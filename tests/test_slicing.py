@@ -294,3 +294,35 @@ def test_llama_8b_sized_layers_sliced_on_the_gpu_keep_their_weights():
     step = ops.w4a16_dequantize_rows(torch.full_like(p2, 0x99999999 - (1 << 32)), s2, torch.arange(nheads * rhd), hidden)
     assert bool(((deq(p2, s2, hidden).float() - kept.float()).abs() <= 0.52 * step.float().abs() + 1e-5).all())
     assert ops.read_and_clear_status("cuda") == 0
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("k_new", [1, 127, 128, 129, 300])
+def test_gpu_row_tiles_and_unaligned_buffers(k_new):
+    """Edges of the 64 x 128 tiles of the row kernel, and source buffers that are only 4- and 2-byte aligned."""
+    from uniql_b200 import ops
+    n_src, n_real, k = 256, 200, 512
+    g = torch.Generator().manual_seed(k_new)
+    packed = torch.randint(-2 ** 31, 2 ** 31 - 1, (k // 16, 2 * n_src), generator=g).to(torch.int32)
+    scale = (torch.rand(k // 128, n_src, generator=g) * 0.01 + 0.001).half()
+    rows = torch.randint(0, k, (k_new,), generator=g)
+    want = qh.w4a16_dequantize(packed, scale)[rows][:, :n_real].t().contiguous()
+    assert torch.equal(ops.w4a16_dequantize_rows(packed.cuda(), scale.cuda(), rows, n_real).cpu(), want)
+    p2 = torch.empty(packed.numel() + 1, dtype=torch.int32, device="cuda")[1:].view_as(packed)
+    s2 = torch.empty(scale.numel() + 1, dtype=torch.half, device="cuda")[1:].view_as(scale)
+    p2.copy_(packed), s2.copy_(scale)
+    assert torch.equal(ops.w4a16_dequantize_rows(p2, s2, rows, n_real).cpu(), want)
+
+
+@pytest.mark.parametrize("reduced", [64, 200, 321, 448, 512])
+def test_up_gate_slice_zeroes_scales_in_place(reduced):
+    """The permuted scales past the kept width against unpermute, zero, permute."""
+    g = torch.Generator().manual_seed(reduced)
+    w = torch.randint(-2 ** 31, 2 ** 31 - 1, (8, 2 * 768), generator=g).to(torch.int32)
+    s = (torch.rand(1, 768, generator=g) + 0.1).half()
+    ws = torch.zeros(768 // 64 * 16, dtype=torch.int32)
+    width = (reduced + 255) // 256 * 256
+    nat = qh.unpermute_group_scales(s[:, :width].contiguous())
+    nat[:, reduced:] = 0
+    got_w, got_s, _ = mh.slice_w4a16_up_gate_proj(w, s, ws, 128, 768, reduced, w.shape)
+    assert torch.equal(got_s, qh.permute_group_scales(nat)) and torch.equal(got_w, w[:, :2 * width])

@@ -128,10 +128,24 @@ def slice_w4a16_up_gate_proj(weight, scale, workspace, hidden_size, intermediate
     assert load_shape[0] == weight.shape[0], "hidden_size dimension mismatch"
     width = _round_up(reduced_intermediate_size, 256)
     assert weight.shape[1] // 2 >= width, "Reduced size shape exceeds recovered weight"
-    packed = weight[:, :2 * width].contiguous()
-    s = unpermute_group_scales(scale[:, :width].contiguous())
-    s[:, reduced_intermediate_size:] = 0
-    return packed, permute_group_scales(s).contiguous(), _workspace(workspace, width)
+    # whole 64-column blocks are 512 bytes: copied as 16-byte elements (contiguous() of int32 columns moves 4 at a time)
+    packed = weight[:, :2 * width]
+    if weight.is_cuda and weight.is_contiguous() and weight.dtype == torch.int32 and weight.shape[1] % 4 == 0 \
+            and weight.data_ptr() % 16 == 0 and weight.storage_offset() % 4 == 0:
+        packed = packed.view(torch.complex128).contiguous().view(torch.int32)
+    else:
+        packed = packed.contiguous()
+    # inside a 64-column block, column i + 8 j sits at 8 i + j: the columns past `reduced` are zeroed where they are stored
+    s = scale[:, :width].clone(memory_format=torch.contiguous_format)
+    blk, rem = divmod(reduced_intermediate_size, 64)
+    if rem:
+        block = s.view(s.shape[0], -1, 8, 8)[:, blk]
+        block[:, :, (rem + 7) // 8:] = 0
+        if rem % 8:
+            block[:, rem % 8:, rem // 8] = 0
+        blk += 1
+    s[:, 64 * blk:] = 0
+    return packed, s, _workspace(workspace, width)
 
 
 def slice_w4a16_down_proj(weight, scale, workspace, hidden_size, intermediate_size, reduced_intermediate_size,

@@ -363,11 +363,12 @@ def w4a16_gather_columns(weight: torch.Tensor, scale: torch.Tensor, col_index: t
     _require_cuda(scale, "scale")
     dev = weight.device
     size_k, n_src_pad = weight.shape[0] * 16, weight.shape[1] // 2
-    idx = col_index.to(device=dev, dtype=torch.int32).contiguous()
-    # load-time call: a synchronising range check is affordable, and the CPU path would raise IndexError here too
-    # (negative entries are allowed: they produce zero columns)
+    # the CPU path would raise IndexError here too (negative entries are allowed: they produce zero columns); an index that
+    # is still on the host is checked there, one on the GPU costs a synchronisation
+    idx = col_index.to(dtype=torch.int32)
     if idx.numel() and int(idx.max()) >= n_src_pad:
         raise RuntimeError("col_index out of range")
+    idx = idx.to(device=dev).contiguous()
     weight, scale = weight.contiguous(), scale.contiguous()
     packed = torch.empty((size_k // 16, 2 * n_out_pad), dtype=torch.int32, device=dev)
     scales = torch.empty((size_k // 128, n_out_pad), dtype=torch.float16, device=dev)
@@ -386,9 +387,10 @@ def w4a16_dequantize_rows(weight: torch.Tensor, scale: torch.Tensor, row_index: 
     _require_cuda(scale, "scale")
     dev = weight.device
     size_k, n_src_pad = weight.shape[0] * 16, weight.shape[1] // 2
-    idx = row_index.to(device=dev, dtype=torch.int32).contiguous()
+    idx = row_index.to(dtype=torch.int32)
     if idx.numel() and (int(idx.min()) < 0 or int(idx.max()) >= size_k):
         raise RuntimeError("row_index out of range")
+    idx = idx.to(device=dev).contiguous()
     weight, scale = weight.contiguous(), scale.contiguous()
     out = torch.empty((n_real, idx.numel()), dtype=torch.float16, device=dev)
     with torch.cuda.device(dev):
