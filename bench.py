@@ -833,7 +833,7 @@ def run_ours(args):
                              "frac_of_measured_bf16_burst": (2.0 * 4096 * n_gate * HIDDEN / (prefill_us * 1e-6) / 1e12)
                              / float(peaks.get("bf16_tflops", 1590.0)),
                              "frac_of_nominal_2250": (2.0 * 4096 * n_gate * HIDDEN / (prefill_us * 1e-6) / 1e12) / 2250.0},
-            "m64_us": {"value": m64_us, "kernel": f"w4a16_gemm_tc_swap_kernel {n_gate}x{HIDDEN} m=64 per GPU",
+            "m64_us": {"value": m64_us, "kernel": f"w4a16_gemm_swap_kernel {n_gate}x{HIDDEN} m=64 per GPU",
                        "weight_gbs": (n_gate * HIDDEN / 2 + n_gate * HIDDEN / 64) / (m64_us * 1e-6) / 1e9},
             "batch_curve": batch_curve,
             "aux_kernels": aux,

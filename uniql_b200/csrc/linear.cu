@@ -1,4 +1,4 @@
-// C-ABI entry points of the W4A16 linear and their regime dispatch (persistent streaming kernel for m <= 16,
+// C-ABI entry points of the W4A16 linear and their regime dispatch (streaming kernel for a few rows,
 // tcgen05 tensor-core kernels above), the grouped decode launch and its tensor-parallel form.
 #include "common.cuh"
 #include "linear_internal.cuh"
