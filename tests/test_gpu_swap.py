@@ -75,3 +75,19 @@ def test_swiglu_pair_and_residual(m, n, k):
     assert torch.equal(got, want)
     (got,) = ops.w4a16_linear_group(x, [g], residual=res)
     assert torch.equal(got, a + res)
+
+
+@pytest.mark.parametrize("m", [5, 16, 17, 64, 256])
+def test_packed_ring_refilled_many_times(m):
+    """Every CTA streams more scale groups than the packed ring has slots (40 and 80 against at most 16), so each slot is
+    handed back and refilled by TMA while other warps still read: a slot released before all lanes of a warp have read it
+    gives wrong weights.  The sums are deterministic, so cold and cached weights must give the same bits."""
+    from uniql_b200 import ops
+    n, k = 148 * 128 + 64, 5120
+    layer = quantized_layer(n + k, n, k)
+    x = make_acts(m, m, k)
+    w, s, b, _ = _dev(layer)
+    first = ops.w4a16_linear(x.cuda(), w, s, b, n)
+    _check(first, x, layer)
+    for _ in range(20):
+        assert torch.equal(ops.w4a16_linear(x.cuda(), w, s, b, n), first)

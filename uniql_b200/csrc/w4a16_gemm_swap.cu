@@ -124,17 +124,6 @@ __device__ __forceinline__ void sw_ld16(uint32_t taddr, uint32_t (&r)[16]) {
 }
 __device__ __forceinline__ void sw_wait_ld() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
 
-// Arrive that cannot be issued before the two registers have been loaded (its predicate depends on them): an arrive does
-// not wait for shared-memory loads in front of it by itself, and a slot handed back too early is refilled under the
-// reader (wrong results with a four-slot ring).  Loads of a warp return in order, so the last pair covers the others.
-__device__ __forceinline__ void sw_arrive_after(uint32_t bar, uint32_t a, uint32_t b) {
-  asm volatile(
-      "{\n\t.reg .pred p;\n\tsetp.lt.u32 p, %1, %2;\n\t"
-      "@p mbarrier.arrive.shared::cta.b64 _, [%0];\n\t@!p mbarrier.arrive.shared::cta.b64 _, [%0];\n\t}"
-      ::"r"(bar), "r"(a), "r"(b)
-      : "memory");
-}
-
 // The eight MMAs of one 128-k stage, the commit that releases the stage, and one poll of the NEXT stage's barrier, in
 // one block: the poll is issued first and its result read last, so its latency hides behind the issue of the MMAs.
 // ("Next": the issuer's next stage.)
@@ -574,7 +563,11 @@ w4a16_gemm_swap_kernel(const __grid_constant__ SwapParams p, const __grid_consta
 #pragma unroll
       for (int kt = 0; kt < 8; ++kt)
         asm volatile("ld.shared.v2.u32 {%0,%1}, [%2];" : "=r"(wq[kt][0]), "=r"(wq[kt][1]) : "r"(pk + kt * 512) : "memory");
-      if (lane == 0) sw_arrive_after(bar_empty_p + 8 * sp, wq[7][0], wq[7][1]);
+      // Every lane has waited in a loop of its own, so lane 0 may be ahead of the others: without the warp barrier its
+      // arrive would hand the slot back, and TMA refill it, under lanes that have yet to read.  The barrier orders all
+      // lanes' reads before the arrive, which releases them to the producer.
+      __syncwarp();
+      if (lane == 0) tc_mbar_arrive(bar_empty_p + 8 * sp);
       if (!timed_out && !tc_mbar_wait(bar_empty + 8 * s, ph ^ 1)) timed_out = true;
       tc_fence_after();
 #pragma unroll
