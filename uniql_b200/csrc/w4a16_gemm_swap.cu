@@ -555,19 +555,12 @@ w4a16_gemm_swap_kernel(const __grid_constant__ SwapParams p, const __grid_consta
         sptr += s_step;
         snext = __ldg(sptr);
       }
-      // The packed words go to registers as soon as they have landed and their slot is handed back at once: a slot that
-      // is held through the conversion (and the wait for the stage) caps the weight stream at ring depth / that time.
       if (!timed_out && !tc_mbar_wait(bar_full_p + 8 * sp, pph)) timed_out = true;
       const uint32_t pk = sbase + OFF_P + sp * P_BYTES + blk_local * P_BLK + lane * 16 + (q & 1) * 8;
       uint32_t wq[8][2];
 #pragma unroll
       for (int kt = 0; kt < 8; ++kt)
         asm volatile("ld.shared.v2.u32 {%0,%1}, [%2];" : "=r"(wq[kt][0]), "=r"(wq[kt][1]) : "r"(pk + kt * 512) : "memory");
-      // Every lane has waited in a loop of its own, so lane 0 may be ahead of the others: without the warp barrier its
-      // arrive would hand the slot back, and TMA refill it, under lanes that have yet to read.  The barrier orders all
-      // lanes' reads before the arrive, which releases them to the producer.
-      __syncwarp();
-      if (lane == 0) tc_mbar_arrive(bar_empty_p + 8 * sp);
       if (!timed_out && !tc_mbar_wait(bar_empty + 8 * s, ph ^ 1)) timed_out = true;
       tc_fence_after();
 #pragma unroll
@@ -602,8 +595,14 @@ w4a16_gemm_swap_kernel(const __grid_constant__ SwapParams p, const __grid_consta
       }
       asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
       tc_fence_before();
+      // One warp barrier in front of both arrives.  The packed slot goes back here, where the stores above have consumed
+      // every lane's words, and not right behind its loads: there the arrive overtook loads still in flight, with a warp
+      // barrier in between too (256 rows, 19008 x 5120: wrong values where TMA refilled the slot under a reader).
       __syncwarp();
-      if (lane == 0) tc_mbar_arrive(bar_full + 8 * s);
+      if (lane == 0) {
+        tc_mbar_arrive(bar_full + 8 * s);
+        tc_mbar_arrive(bar_empty_p + 8 * sp);
+      }
       s += p.nsets;
       if (s >= p.nst) { s -= p.nst; ph ^= 1; }
       sp += p.nsets;
