@@ -112,3 +112,40 @@ def test_tensor_parallel_launches_replay_from_a_cuda_graph(comm):
         torch.cuda.synchronize()
         assert torch.equal(y, want)
     assert ops.read_and_clear_status("cuda") == 0
+
+
+@pytest.mark.parametrize("m", [4, 5, 8, 16])
+@pytest.mark.parametrize("n,k", [(128, 128), (192, 1152), (4096, 4096), (16384, 256)])
+def test_sum_over_one_rank_has_the_bits_of_the_plain_launch(comm, m, n, k):
+    """Both sides of the row count at which the kernel changes, one scale group, a half-empty tile, a tile shared by a
+    cluster, one CTA per tile.  Without bias and residual the only rounding of the exchanged partial is the plain launch's
+    own, so nothing may differ."""
+    from uniql_b200 import ops
+    p, s, _ = _dev(quantized_layer(n + k, n, k))
+    for rep in range(3):
+        x = make_acts(m + rep, m, k).cuda()
+        got = comm.linear_all_reduce(x, p, s, None, n)
+        (want,) = ops.w4a16_linear_group(x, [(p, s, None, n)])
+        torch.cuda.synchronize()
+        assert torch.equal(got, want)
+    assert ops.read_and_clear_status("cuda") == 0
+
+
+@pytest.mark.parametrize("m", [4, 5, 16])
+@pytest.mark.parametrize("hidden,inter", [(2048, 2048), (256, 16384)])
+def test_gathered_chain_on_split_and_on_repeated_tiles(comm, m, hidden, inter):
+    """Pair tiles that a cluster shares, and more pair tiles than SMs; the down projection reads the row from the feature
+    area, so a word that is missing or misplaced shows up in its result."""
+    from uniql_b200 import ops
+    (gp, gs, _), (up_, us, _), (dp, ds, _) = (_dev(quantized_layer(i + inter, *shape)) for i, shape in
+                                              enumerate([(inter, hidden), (inter, hidden), (hidden, inter)]))
+    for rep in range(3):
+        x = make_acts(10 + rep, m, hidden).cuda()
+        h = comm.gate_up_gather(x, (gp, gs, None, inter), (up_, us, None, inter), 0)
+        y = comm.down_gather_reduce(m, (dp, ds, None, hidden), inter, 0)
+        (h0,) = ops.w4a16_linear_group(x, [(gp, gs, None, inter), (up_, us, None, inter)], epilogue="swiglu")
+        (y0,) = ops.w4a16_linear_group(h0, [(dp, ds, None, hidden)], hadamard_dim=inter)
+        torch.cuda.synchronize()
+        assert torch.equal(h, h0)
+        assert torch.allclose(y.float(), y0.float(), rtol=1e-3, atol=1e-3 * float(y0.float().abs().max()))
+    assert ops.read_and_clear_status("cuda") == 0

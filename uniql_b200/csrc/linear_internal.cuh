@@ -91,6 +91,7 @@ struct SwapArgs {
   int64_t ldr;
   const __half* A;
   int64_t lda, m;
+  const CommView* comm;       // at most 16 rows: the exchanges of a tensor-parallel step; nullptr: single GPU
 };
 bool gemm_swap_supported(int64_t m, int64_t k, const int64_t* n, int nproj);
 int launch_gemm_swap(const SwapArgs& a, cudaStream_t stream);

@@ -1,14 +1,14 @@
-// Decode-regime W4A16 linear (m <= 16) for sm_100a: the dispatch between the two decode kernels, the entry point that
-// needs no caller scratch, and the second of the two kernels -- a persistent, slot-balanced, weight-streaming skinny GEMM.
+// Decode-regime W4A16 linear (m <= 16) for sm_100a: the dispatch between the kernels that run it, the entry point that
+// needs no caller scratch, and one of these kernels -- a persistent, slot-balanced, weight-streaming skinny GEMM.
 //
-// Both kernels replace the small-batch instantiations of UniQL's Marlin kernel
+// The kernels replace the small-batch instantiations of UniQL's Marlin kernel
 // (csrc/linear/marlin_gemm_kernel.cuh:176-740, tile table :792-800) while consuming the very same
 // packed buffers (quantize/quantize_helpers.py:145-165 weight order, :54-62 scale order), and the separate
 // launches the reference's blocks make around it: gate_proj / up_proj / act_fn(gate) * up
 // (modeling/llama/llama_qblocks.py:48-51), q/k/v (:104-106), the residual add, and the online Hadamard in front of
 // down_proj / out_proj (quantize/quant_hadamard_layers.py:16-18).  launch_decode() sends a launch to the CTA-tiled kernel
-// of w4a16_gemv.cu (the default, and the only one that talks to other GPUs) or, with UNIQL_B200_DECODE_ENGINE=slot, to
-// the kernel below (single GPU).
+// of w4a16_gemv.cu (few rows) or the operand-swapped tensor-core kernel of w4a16_gemm_swap.cu, both of which also talk to
+// other GPUs, or, with UNIQL_B200_DECODE_ENGINE=slot, to the kernel below (single GPU).
 //
 // How the packed layout is consumed.  Packed row kt (16 k-values) holds, for every 64-column block,
 // 512 contiguous bytes; lane i of a warp owns bytes 16i..16i+15 = four words j=0..3.  With g = i/4 and
@@ -1085,10 +1085,26 @@ static int launch_variant(const DecodeParams& p, const DecodePlan& pl, cudaStrea
 
 constexpr int kSwapMinRows = 5;
 
+// What the exchange areas of a communicator have room for.
+static int comm_fits(const DecodeArgs& a) {
+  int64_t blocks = 0;
+  for (int i = 0; i < a.nproj; ++i) blocks += a.proj[i].n / 64;
+  const bool pair = a.epilogue == UNIQL_EPILOGUE_SWIGLU;
+  if (a.comm->reduce && (pair || a.nproj != 1)) return UNIQL_EINVAL;
+  if (a.comm->reduce && blocks > a.comm->block_cap) return UNIQL_ESHAPE;
+  const int64_t units = pair ? blocks / 2 : blocks;
+  if (a.comm->gather_out && (a.comm->col_offset % 64 || a.comm->col_offset + units * 64 > a.comm->feat_cap)) return UNIQL_ESHAPE;
+  return UNIQL_OK;
+}
+
 int launch_decode(const DecodeArgs& a, cudaStream_t stream) {
   int64_t n[kMaxProj] = {0, 0, 0, 0};
   if (a.nproj < 1 || a.nproj > kMaxProj) return UNIQL_EINVAL;
   for (int i = 0; i < a.nproj; ++i) n[i] = a.proj[i].n;
+  if (a.comm) {
+    const int st = comm_fits(a);
+    if (st != UNIQL_OK) return st;
+  }
   if (!use_slot_engine(a)) {
     // CTA-tiled kernel; an online Hadamard runs as its own kernel in front (rows rounded to fp16 in scratch) and the
     // linear's weight stream overlaps it through the programmatic dependent launch
@@ -1115,11 +1131,12 @@ int launch_decode(const DecodeArgs& a, cudaStream_t stream) {
       if (st != UNIQL_OK) return st;
       lda = a.hadamard_dim;
     }
-    // From five rows on the tensor-core kernel with exact codes as the operand and fp32 group scales (the arithmetic of the
+    // From five rows on, with and without a communicator (a step of a tensor-parallel layer has the sums of the plain
+    // launch), the tensor-core kernel with exact codes as the operand and fp32 group scales (the arithmetic of the
     // tiled kernel) is faster: its work per weight does not grow with the rows, while the tiled kernel stages rows x k
     // activations in every CTA.  14336 x 4096 in us, tiled / tensor core: 4 rows 9.8 / 11.4, 8 rows 12.8 / 11.7, 16 rows
     // 18.6 / 11.7; 4096 x 14336: 11.8 / 12.6, 13.9 / 12.7, 18.7 / 12.8; 4096 x 4096: 6.7 / 7.6, 7.1 / 7.5, 8.5 / 7.6.
-    if (!a.comm && a.m >= kSwapMinRows && gemm_swap_supported(a.m, a.k, n, a.nproj)) {
+    if (a.m >= kSwapMinRows && gemm_swap_supported(a.m, a.k, n, a.nproj)) {
       LinearArgs la[kMaxProj];
       void* ds[kMaxProj];
       for (int i = 0; i < a.nproj; ++i) {
@@ -1131,6 +1148,7 @@ int launch_decode(const DecodeArgs& a, cudaStream_t stream) {
       SwapArgs sa{};
       sa.projs = la; sa.Ds = ds; sa.nproj = a.nproj; sa.pair = a.epilogue == UNIQL_EPILOGUE_SWIGLU;
       sa.residual = a.residual; sa.ldr = a.ldr; sa.A = Ain; sa.lda = lda; sa.m = a.m;
+      sa.comm = a.comm;
       return launch_gemm_swap(sa, stream);
     }
     return launch_gemv_group(a, Ain, lda, stream);

@@ -30,12 +30,19 @@
 // With few tiles a cluster of up to 8 CTAs shares each tile, every CTA reducing a slice of k; the partial accumulators
 // are parked in shared memory and summed in rank order through distributed shared memory (deterministic).
 //
+// TP (at most 16 rows): the launch is a step of a tensor-parallel layer.  The sums are those of the plain launch; the
+// epilogue works on four columns of a row at a time and carries the exchanges of tp_exchange.cuh: the sum of a row-parallel
+// shard over the ranks, or the columns of a column shard stored into every rank's feature area.  A CTA pushes all its words
+// of a tile before it waits for any, and every rank takes its tiles in ascending order (the tiled kernel too, which a rank
+// with another k may run), so the lowest unfinished tile never waits for a higher one; waits are bounded.
+//
 // Bound: weight stream (HBM) below ~128 rows, tensor pipe above; in practice the per-stage chain of the dequantise warps
 // (~260 issued instructions per warp and stage) and the fixed cost of a launch.
 // Every mbarrier wait is bounded; a wait that gives up sets UNIQL_STATUS_WAIT_TIMEOUT and the kernel drains.
 #include "common.cuh"
 #include "linear_internal.cuh"
 #include "tc.cuh"
+#include "tp_exchange.cuh"
 
 #include <cuda.h>
 #include <stdlib.h>
@@ -86,6 +93,7 @@ struct SwapParams {
   int nbuf;                                     // tiles whose accumulators are kept (1 or 2)
   int off_x;                                    // activation ring in shared memory
   int* status_word;
+  CommView cv;                                  // tensor-parallel launches only
 };
 struct SwapMaps {
   CUtensorMap w[kMaxProj];                      // packed weights, boxes of 128 words x 8 packed rows
@@ -215,17 +223,40 @@ __device__ __forceinline__ void sw_finish4(const SwOut& o, int row, int c4, floa
   }
 }
 
+// The same quad of a tensor-parallel launch (u: the up columns of a pair): like sw_value, and a column shard's columns
+// travel to every rank's feature area.
+template <bool PAIR>
+__device__ __forceinline__ void sw_finish4_tp(const SwOut& o, const CommView& cv, uint32_t gather_ep, int row, int c4,
+                                              float4 v, float4 u) {
+  const int n = o.n0 + c4;
+  if (n >= o.n_out || row >= o.row_end) return;
+  __half* d = o.D + (size_t)row * o.ldd + n;
+  const float a[4] = {v.x, v.y, v.z, v.w}, b[4] = {u.x, u.y, u.z, u.w};
+  __half h[4];
+#pragma unroll
+  for (int e = 0; e < 4; ++e) {
+    h[e] = __float2half_rn(0.f);
+    if (n + e < o.n_out) d[e] = h[e] = sw_value<PAIR>(o, row, n + e, a[e], b[e]);
+  }
+  if (cv.gather_out) tp_feature4(cv, gather_ep, row, n, o.n_out, h);
+}
+
+__device__ __forceinline__ float4 sw_lds_f4(uint32_t addr) {
+  const uint4 v = tc_lds128(addr);
+  return make_float4(__uint_as_float(v.x), __uint_as_float(v.y), __uint_as_float(v.z), __uint_as_float(v.w));
+}
 __device__ __forceinline__ float sw_lds_f(uint32_t addr) {
   float v;
   asm volatile("ld.shared.f32 %0, [%1];" : "=f"(v) : "r"(addr) : "memory");
   return v;
 }
 
-template <bool GS, bool PAIR>
+template <bool GS, bool PAIR, bool TP>
 __global__ void __launch_bounds__(sw::THREADS, 1)
 w4a16_gemm_swap_kernel(const __grid_constant__ SwapParams p, const __grid_constant__ CUtensorMap xmap,
                        const __grid_constant__ SwapMaps wmaps) {
   using namespace sw;
+  static_assert(GS || !TP, "the exchanges have room for 16 rows");
   extern __shared__ uint8_t smem_unaligned[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_unaligned) + 1023) & ~(uintptr_t)1023);
   const uint32_t sbase = tc_smem_addr(smem);
@@ -299,6 +330,40 @@ w4a16_gemm_swap_kernel(const __grid_constant__ SwapParams p, const __grid_consta
   const uint32_t tmem_base = *tmem_slot;
   bool timed_out = false;
 
+  // TP: finishes rows [r0, r1) of a tile with `nthreads` threads, four columns of a row per thread and step; `quad` delivers
+  // the sums of four adjacent columns of the tile.  kQuads divides every nthreads, so a thread stays in one 64-column block.
+  auto finish_tp = [&](const SwOut& o, int r0, int r1, int tid, int nthreads, uint32_t reduce_ep, uint32_t gather_ep, auto&& quad) {
+    constexpr int kQuads = PAIR ? 16 : 32;
+    const int c4 = (tid % kQuads) * 4, block = (o.n0 + c4) >> 6, c = c4 & 63;
+    const bool push = !PAIR && p.cv.reduce;
+    if (o.n0 + c4 >= p.proj[0].N && push) return;   // past the packed width: nothing travels (a reduce launch has one projection)
+    if (push) {
+#pragma unroll 1
+      for (int r = r0 + tid / kQuads; r < r1; r += nthreads / kQuads) tp_push4(p.cv, reduce_ep, block, o.row0 + r, c, quad(r, c4));
+    }
+#pragma unroll 1
+    for (int r = r0 + tid / kQuads; r < r1; r += nthreads / kQuads) {
+      const float4 v = push ? tp_gather4<4>(p.cv, reduce_ep, block, o.row0 + r, c, timed_out) : quad(r, c4);
+      const float4 u = PAIR ? quad(r, c4 + 64) : make_float4(0.f, 0.f, 0.f, 0.f);
+      sw_finish4_tp<PAIR>(o, p.cv, gather_ep, o.row0 + r, c4, v, u);
+    }
+  };
+  // Epochs of this thread's words (see finish_tp).  The wait keeps every exchange of this launch behind the preceding ones:
+  // they advance the counters, and a peer that runs one exchange ahead relies on this rank having finished the one before.
+  auto tp_epochs = [&](const SwOut& o, int tid, uint32_t& reduce_ep, uint32_t& gather_ep) {
+    pdl_wait();
+    const int n = o.n0 + (tid % (PAIR ? 16 : 32)) * 4;
+    reduce_ep = (p.cv.reduce && n < p.proj[0].N) ? *tp_reduce_counter(p.cv, n >> 6) + 1 : 0;
+    gather_ep = p.cv.gather_out ? tp_gather_epoch(p.cv) : 0;
+  };
+  // once every thread has finished its part of the tile: one thread per 64-column block
+  auto tp_advance = [&](const SwOut& o, int tid) {
+    if (p.cv.reduce && tid < 2 && o.n0 + tid * 64 < p.proj[0].N) {
+      volatile uint32_t* ctr = tp_reduce_counter(p.cv, (o.n0 >> 6) + tid);
+      *ctr = *ctr + 1;
+    }
+  };
+
   // Finishes 16 rows of a tile, held by four warps (one per quarter of the columns; `v`: this lane's column).  A cluster
   // parks them in the activation ring (idle once the last MMA has completed) for the sum over the ranks, below.
   // Otherwise the values of a plain launch are stored straight from the registers (64 bytes per warp and row); a pair
@@ -308,6 +373,16 @@ w4a16_gemm_swap_kernel(const __grid_constant__ SwapParams p, const __grid_consta
     if (p.split > 1) {
 #pragma unroll
       for (int e = 0; e < RC; ++e) tc_sts32(xbase + (c0 + e) * ROW_BYTES + col * 4, __float_as_uint(v[e]));
+    } else if (TP) {
+      uint32_t reduce_ep, gather_ep;
+      tp_epochs(o, gtid, reduce_ep, gather_ep);
+#pragma unroll
+      for (int e = 0; e < RC; ++e) tc_sts32(park + e * ROW_BYTES + col * 4, __float_as_uint(v[e]));
+      asm volatile("bar.sync %0, 128;" ::"r"(bar) : "memory");
+      finish_tp(o, 0, min(RC, o.row_end - o.row0), gtid, 128, reduce_ep, gather_ep,
+                [&](int r, int c) { return sw_lds_f4(park + r * ROW_BYTES + c * 4); });
+      asm volatile("bar.sync %0, 128;" ::"r"(bar) : "memory");
+      tp_advance(o, gtid);
     } else if (!PAIR) {
       const int n = o.n0 + col, rows = o.row_end - o.row0 - c0;
       if (n < o.n_out) {
@@ -629,13 +704,38 @@ w4a16_gemm_swap_kernel(const __grid_constant__ SwapParams p, const __grid_consta
     const bool have = warp >= FIRST_EPI_WARP && tile0 < p.ntiles;
     SwOut o;
     if (have) o = sw_out_of(p, tile0);
+    uint32_t reduce_ep = 0, gather_ep = 0;
+    if (TP && have) tp_epochs(o, (int)threadIdx.x - FIRST_EPI_WARP * 32, reduce_ep, gather_ep);
     __syncwarp();
     sw_cluster_sync();                          // every rank's partial tile is in its shared memory
     if (have) {
       const int ftid = (int)threadIdx.x - FIRST_EPI_WARP * 32;
       const int rows = min(p.Mb, p.M - o.row0);
       const int row0 = rows * rank / p.split, row1 = rows * (rank + 1) / p.split;
-      if (PAIR) {
+      // the sums of four adjacent columns: the quads of every rank, added in rank order
+      auto sum4 = [&](int r, int c4) {
+        const uint32_t off = (uint32_t)r * ROW_BYTES + c4 * 4;
+        float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll 1
+        for (int r0 = 0; r0 < p.split; r0 += 4) {
+          float4 t[4];
+#pragma unroll
+          for (int i = 0; i < 4; ++i)
+            if (r0 + i < p.split) {
+              uint32_t remote;
+              asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote) : "r"(xbase + off), "r"(r0 + i));
+              asm volatile("ld.shared::cluster.v4.f32 {%0,%1,%2,%3}, [%4];"
+                           : "=f"(t[i].x), "=f"(t[i].y), "=f"(t[i].z), "=f"(t[i].w) : "r"(remote) : "memory");
+            }
+#pragma unroll
+          for (int i = 0; i < 4; ++i)
+            if (r0 + i < p.split) { v.x += t[i].x; v.y += t[i].y; v.z += t[i].z; v.w += t[i].w; }
+        }
+        return v;
+      };
+      if (TP) {
+        finish_tp(o, row0, row1, ftid, FINISH_THREADS, reduce_ep, gather_ep, sum4);
+      } else if (PAIR) {
         auto sum_ranks = [&](uint32_t off) {
           float t[8], v = 0.f;
 #pragma unroll
@@ -664,29 +764,13 @@ w4a16_gemm_swap_kernel(const __grid_constant__ SwapParams p, const __grid_consta
 #pragma unroll 1
         for (int idx = ftid; idx < (row1 - row0) * 32; idx += FINISH_THREADS) {
           const int r = row0 + (idx >> 5), c4 = (idx & 31) * 4;
-          const uint32_t off = (uint32_t)r * ROW_BYTES + c4 * 4;
-          float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-#pragma unroll 1
-          for (int r0 = 0; r0 < p.split; r0 += 4) {
-            float4 t[4];
-#pragma unroll
-            for (int i = 0; i < 4; ++i)
-              if (r0 + i < p.split) {
-                uint32_t remote;
-                asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote) : "r"(xbase + off), "r"(r0 + i));
-                asm volatile("ld.shared::cluster.v4.f32 {%0,%1,%2,%3}, [%4];"
-                             : "=f"(t[i].x), "=f"(t[i].y), "=f"(t[i].z), "=f"(t[i].w) : "r"(remote) : "memory");
-              }
-#pragma unroll
-            for (int i = 0; i < 4; ++i)
-              if (r0 + i < p.split) { v.x += t[i].x; v.y += t[i].y; v.z += t[i].z; v.w += t[i].w; }
-          }
-          sw_finish4(o, o.row0 + r, c4, v);
+          sw_finish4(o, o.row0 + r, c4, sum4(r, c4));
         }
       }
     }
     __syncwarp();
     sw_cluster_sync();                          // no rank leaves while its shared memory may still be read
+    if (TP && have && rank == 0) tp_advance(o, (int)threadIdx.x - FIRST_EPI_WARP * 32);
   }
   if (timed_out && p.status_word) atomicOr(p.status_word, UNIQL_STATUS_WAIT_TIMEOUT);
   tc_fence_before();
@@ -704,9 +788,10 @@ static int swap_env(const char* name, int dflt) {
 }
 
 typedef void (*SwapKernel)(const SwapParams, const CUtensorMap, const SwapMaps);
-static SwapKernel swap_kernel(bool gs, bool pair) {
-  if (gs) return pair ? w4a16_gemm_swap_kernel<true, true> : w4a16_gemm_swap_kernel<true, false>;
-  return pair ? w4a16_gemm_swap_kernel<false, true> : w4a16_gemm_swap_kernel<false, false>;
+static SwapKernel swap_kernel(bool gs, bool pair, bool tp) {
+  if (tp) return pair ? w4a16_gemm_swap_kernel<true, true, true> : w4a16_gemm_swap_kernel<true, false, true>;
+  if (gs) return pair ? w4a16_gemm_swap_kernel<true, true, false> : w4a16_gemm_swap_kernel<true, false, false>;
+  return pair ? w4a16_gemm_swap_kernel<false, true, false> : w4a16_gemm_swap_kernel<false, false, false>;
 }
 
 // Clusters of `split` CTAs that can be resident together (0 if the query fails).
@@ -729,7 +814,7 @@ static int swap_max_clusters(bool gs, int split, int smem) {
   cfg.attrs = attr;
   cfg.numAttrs = 1;
   int n = 0;
-  if (cudaOccupancyMaxActiveClusters(&n, swap_kernel(gs, false), &cfg) != cudaSuccess) {
+  if (cudaOccupancyMaxActiveClusters(&n, swap_kernel(gs, false, false), &cfg) != cudaSuccess) {
     (void)cudaGetLastError();
     n = 0;
   }
@@ -818,9 +903,9 @@ static SwapShape swap_shape(int64_t m, int64_t k, int ctiles, bool gs) {
 }
 
 // The model's figure for a launch of `ctiles` 128-column tiles (the kernel's attributes must have been set: see there).
-static int swap_set_attributes(bool gs, bool pair);
+static int swap_set_attributes(bool gs, bool pair, bool tp);
 double gemm_swap_cycles(int64_t m, int64_t k, int ctiles) {
-  if (swap_set_attributes(m <= 16, false) != UNIQL_OK) return 1e30;
+  if (swap_set_attributes(m <= 16, false, false) != UNIQL_OK) return 1e30;
   return swap_shape(m, k, ctiles, m <= 16).cycles;
 }
 
@@ -832,15 +917,16 @@ bool gemm_swap_supported(int64_t m, int64_t k, const int64_t* n, int nproj) {
 }
 
 // Function attributes are per device; the occupancy query behind the k-split needs them too (always on the plain kernel).
-static int swap_set_attributes(bool gs, bool pair) {
-  static thread_local bool set[64][4] = {};
+static int swap_set_attributes(bool gs, bool pair, bool tp) {
+  static thread_local bool set[64][8] = {};
   int dev = 0;
   cudaGetDevice(&dev);
   if (dev < 0 || dev >= 64) dev = 0;
-  for (int pr = 0; pr <= (pair ? 1 : 0); ++pr) {
-    bool& done = set[dev][(gs ? 2 : 0) + pr];
+  for (int own = 0; own < 2; ++own) {
+    const bool pr = own && pair, t = own && tp;
+    bool& done = set[dev][(gs ? 4 : 0) + (pr ? 2 : 0) + (t ? 1 : 0)];
     if (done) continue;
-    UNIQL_CUDA_TRY(cudaFuncSetAttribute(swap_kernel(gs, pr != 0), cudaFuncAttributeMaxDynamicSharedMemorySize, sw::SMEM_MAX));
+    UNIQL_CUDA_TRY(cudaFuncSetAttribute(swap_kernel(gs, pr, t), cudaFuncAttributeMaxDynamicSharedMemorySize, sw::SMEM_MAX));
     done = true;
   }
   return UNIQL_OK;
@@ -874,8 +960,12 @@ int launch_gemm_swap(const SwapArgs& a, cudaStream_t stream) {
   p.nproj = a.nproj;
   p.residual = (const __half*)a.residual; p.ldr = a.ldr;
   const bool gs = m <= 16;
+  if (a.comm) {
+    if (!gs || (a.comm->reduce && (a.nproj != 1 || a.pair))) return UNIQL_EINVAL;
+    p.cv = *a.comm;
+  }
   {
-    const int st = swap_set_attributes(gs, a.pair);
+    const int st = swap_set_attributes(gs, a.pair, a.comm != nullptr);
     if (st != UNIQL_OK) return st;
   }
   const SwapShape shape = swap_shape(m, k, ctiles, gs);
@@ -925,7 +1015,7 @@ int launch_gemm_swap(const SwapArgs& a, cudaStream_t stream) {
   }
   cfg.attrs = attr;
   cfg.numAttrs = nattr;
-  UNIQL_CUDA_TRY(cudaLaunchKernelEx(&cfg, swap_kernel(gs, a.pair), p, xmap, wmaps));
+  UNIQL_CUDA_TRY(cudaLaunchKernelEx(&cfg, swap_kernel(gs, a.pair, a.comm != nullptr), p, xmap, wmaps));
   return launch_status();
 }
 

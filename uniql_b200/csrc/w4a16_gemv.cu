@@ -1,4 +1,4 @@
-// Decode-regime W4A16 linear (m <= 16; without tensor parallelism used up to 4 rows) for sm_100a: a weight-streaming skinny GEMM.
+// Decode-regime W4A16 linear (m <= 16; launch_decode uses it up to 4 rows) for sm_100a: a weight-streaming skinny GEMM.
 //
 // Replaces the small-batch instantiations of UniQL's Marlin kernel
 // (csrc/linear/marlin_gemm_kernel.cuh:176-740, tile table :792-800) while consuming the very same
@@ -36,6 +36,7 @@
 #include "common.cuh"
 #include "linear_internal.cuh"
 #include "tma.cuh"
+#include "tp_exchange.cuh"
 
 #include <cuda.h>
 #include <stdlib.h>
@@ -88,20 +89,6 @@ struct GemvParams {
   int npf;
   CommView cv;          // tensor parallelism: cross-GPU sum of a row-parallel shard / feature gather of a column shard
 };
-
-constexpr int kGemvSpinLimit = 1 << 22;   // polls of a word another GPU has to write before giving up
-
-__device__ __forceinline__ void gemv_st_word(uint2* p, uint32_t data, uint32_t flag) {
-  asm volatile("st.relaxed.sys.global.v2.u32 [%0], {%1, %2};" ::"l"(p), "r"(data), "r"(flag) : "memory");
-}
-__device__ __forceinline__ uint4 gemv_ld_word2(const uint2* p) {   // two adjacent {data, epoch} words
-  uint4 v;
-  asm volatile("ld.relaxed.sys.global.v4.u32 {%0, %1, %2, %3}, [%4];"
-               : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w)
-               : "l"(p)
-               : "memory");
-  return v;
-}
 
 // virtual block -> (projection, block inside it)
 __device__ __forceinline__ void gemv_proj_of(const GemvParams& p, int vb, int& pi, int& lb) {
@@ -275,16 +262,11 @@ w4a16_gemv_kernel(const __grid_constant__ GemvParams p) {
   pdl_launch_dependents();
   pdl_wait();
   if ((p.cv.reduce || p.cv.gather_out) && tid < p.WN) {
-    // epoch counters live on the device (CUDA-graph replay safe), one per 64-column block (per gate/up pair)
+    // one per 64-column block (per gate/up pair); read behind the wait: the preceding launch may have advanced them
     const int vb = blockIdx.x * p.WN + tid;
     if (vb < p.nblk) {
-      const size_t unit = (size_t)(p.swiglu ? vb >> 1 : vb);
-      if (p.cv.reduce)
-        s_repoch[tid] = *reinterpret_cast<const volatile uint32_t*>(p.cv.bufs[p.cv.rank] + p.cv.reduce_epoch_off + 4 * unit) + 1;
-      // feature gather: one epoch per launch (this rank's gather counter + 1); the counter itself is advanced by the
-      // consumer of the gathered row (hadamard_split_feat_kernel), which runs between two producer launches
-      if (p.cv.gather_out)
-        s_gepoch[tid] = *reinterpret_cast<const volatile uint32_t*>(p.cv.bufs[p.cv.rank] + p.cv.gather_epoch_off) + 1;
+      if (p.cv.reduce) s_repoch[tid] = *tp_reduce_counter(p.cv, p.swiglu ? vb >> 1 : vb) + 1;
+      if (p.cv.gather_out) s_gepoch[tid] = tp_gather_epoch(p.cv);
     }
   }
 
@@ -511,19 +493,7 @@ w4a16_gemv_kernel(const __grid_constant__ GemvParams p) {
       }
       if (p.residual) h[e] = __float2half_rn(__half2float(h[e]) + __half2float(p.residual[(size_t)m * p.ldr + n + e]));
     }
-    if (p.cv.gather_out) {
-      // column shard of a tensor-parallel layer: the finished columns also go, as epoch-tagged words, into every rank's
-      // feature area (only real columns travel; n_out is even)
-      const uint32_t ep = s_gepoch[(nv - n_base) >> 6];
-      const size_t word = ((size_t)(ep & 1u) * 16 + m) * (size_t)(p.cv.feat_cap >> 1) + (size_t)((p.cv.col_offset + n) >> 1);
-      const uint32_t w0 = (uint32_t)__half_as_ushort(h[0]) | ((uint32_t)__half_as_ushort(h[1]) << 16);
-      const uint32_t w1 = (uint32_t)__half_as_ushort(h[2]) | ((uint32_t)__half_as_ushort(h[3]) << 16);
-      for (int r = 0; r < p.cv.world; ++r) {
-        uint2* dst = reinterpret_cast<uint2*>(p.cv.bufs[r] + p.cv.gather_off) + word;
-        if (n + 1 < pr.n_out) gemv_st_word(dst, w0, ep);
-        if (n + 3 < pr.n_out) gemv_st_word(dst + 1, w1, ep);
-      }
-    }
+    if (p.cv.gather_out) tp_feature4(p.cv, s_gepoch[(nv - n_base) >> 6], m, n, pr.n_out, h);
     __half* d = pr.D + (size_t)m * pr.ldd + n;
     if (n + 3 < pr.n_out && ((reinterpret_cast<uintptr_t>(d) & 7u) == 0)) {
       uint2 pk;
@@ -537,52 +507,14 @@ w4a16_gemv_kernel(const __grid_constant__ GemvParams p) {
     }
   };
 
-  // Row-parallel shard of a tensor-parallel layer: where a rank would store its fp16 result it stores the partial, as
-  // epoch-tagged words, into every rank's staging block (addressed per 64-column block: 16 rows x 32 words) ...
+  // Row-parallel shard of a tensor-parallel layer: the partial goes out to every rank, then what arrived is added up.
   bool wait_failed = false;
   auto push4 = [&](int m, int nv, float4 v) {
-    const int vb = nv >> 6;
-    if (vb >= p.nblk) return;
-    const uint32_t ep = s_repoch[(nv - n_base) >> 6];
-    const __half2 lo = __floats2half2_rn(v.x, v.y), hi = __floats2half2_rn(v.z, v.w);
-    const size_t word = (size_t)vb * kFuseBlockWords + (size_t)m * 32 + ((nv & 63) >> 1);
-    const size_t slot = ((size_t)(ep & 1u) * p.cv.world + p.cv.rank) * (size_t)p.cv.block_cap * kFuseBlockWords + word;
-    for (int r = 0; r < p.cv.world; ++r) {
-      uint2* dst = reinterpret_cast<uint2*>(p.cv.bufs[r] + p.cv.reduce_off) + slot;
-      gemv_st_word(dst, *reinterpret_cast<const uint32_t*>(&lo), ep);
-      gemv_st_word(dst + 1, *reinterpret_cast<const uint32_t*>(&hi), ep);
-    }
+    if ((nv >> 6) < p.nblk) tp_push4(p.cv, s_repoch[(nv - n_base) >> 6], nv >> 6, m, nv & 63, v);
   };
-  // ... and then adds up the words of all ranks that arrived in its own block (bounded wait, rank order, fp32: the same
-  // bits on every rank)
   auto gather4 = [&](int m, int nv) {
-    float4 acc4 = make_float4(0.f, 0.f, 0.f, 0.f);
-    const int vb = nv >> 6;
-    if (vb >= p.nblk) return acc4;
-    const uint32_t ep = s_repoch[(nv - n_base) >> 6];
-    const size_t word = (size_t)vb * kFuseBlockWords + (size_t)m * 32 + ((nv & 63) >> 1);
-    const uint2* base = reinterpret_cast<const uint2*>(p.cv.bufs[p.cv.rank] + p.cv.reduce_off) +
-                        (size_t)(ep & 1u) * p.cv.world * (size_t)p.cv.block_cap * kFuseBlockWords + word;
-    // the first look at every rank's words goes out together (one round trip instead of one per rank); a word that
-    // has not arrived yet is then polled on its own
-    const size_t rstride = (size_t)p.cv.block_cap * kFuseBlockWords;
-    uint4 w[8];
-#pragma unroll
-    for (int r = 0; r < 8; ++r)
-      if (r < p.cv.world) w[r] = gemv_ld_word2(base + (size_t)r * rstride);
-#pragma unroll
-    for (int r = 0; r < 8; ++r)
-      if (r < p.cv.world) {
-        int spin = 0;
-        while ((w[r].y != ep || w[r].w != ep) && !wait_failed) {
-          if (++spin > kGemvSpinLimit) { wait_failed = true; break; }
-          w[r] = gemv_ld_word2(base + (size_t)r * rstride);
-        }
-        const float2 a = __half22float2(*reinterpret_cast<const __half2*>(&w[r].x));
-        const float2 b = __half22float2(*reinterpret_cast<const __half2*>(&w[r].z));
-        acc4.x += a.x; acc4.y += a.y; acc4.z += b.x; acc4.w += b.y;
-      }
-    return acc4;
+    if ((nv >> 6) >= p.nblk) return make_float4(0.f, 0.f, 0.f, 0.f);
+    return tp_gather4<8>(p.cv, s_repoch[(nv - n_base) >> 6], nv >> 6, m, nv & 63, wait_failed);
   };
   // finishes output items [i0, i1) whose values `sumfn(m, col)` delivers
   auto finish_items = [&](int i0, int i1, auto&& sumfn) {
@@ -615,8 +547,7 @@ w4a16_gemv_kernel(const __grid_constant__ GemvParams p) {
     if (p.cv.reduce && tid < p.WN) {
       const int vb = blockIdx.x * p.WN + tid;
       if (vb < p.nblk) {
-        const size_t unit = (size_t)(p.swiglu ? vb >> 1 : vb);
-        *reinterpret_cast<volatile uint32_t*>(p.cv.bufs[p.cv.rank] + p.cv.reduce_epoch_off + 4 * unit) = s_repoch[tid];
+        *tp_reduce_counter(p.cv, p.swiglu ? vb >> 1 : vb) = s_repoch[tid];
       }
     }
   };
@@ -920,13 +851,7 @@ int launch_gemv_group(const DecodeArgs& a, const __half* A, int64_t lda, cudaStr
   p.partials = (float*)((char*)a.scratch + UNIQL_SCRATCH_COUNTER_BYTES);
   const int grid_x = (p.nblk + p.WN - 1) / p.WN;
   if ((size_t)grid_x * sizeof(int) > UNIQL_SCRATCH_COUNTER_BYTES) return UNIQL_ESHAPE;
-  if (a.comm) {
-    p.cv = *a.comm;
-    if (p.cv.reduce && (a.epilogue != UNIQL_EPILOGUE_NONE || a.nproj != 1)) return UNIQL_EINVAL;
-    if (p.cv.reduce && vb > p.cv.block_cap) return UNIQL_ESHAPE;
-    const int units = pair ? vb / 2 : vb;
-    if (p.cv.gather_out && (p.cv.col_offset % 64 || p.cv.col_offset + (int64_t)units * 64 > p.cv.feat_cap)) return UNIQL_ESHAPE;
-  }
+  if (a.comm) p.cv = *a.comm;
   p.npf = 0;
   for (int i = 0; i < a.nprefetch && i < 4; ++i)
     if (a.prefetch_ptr[i] && a.prefetch_bytes[i] >= 128) {
