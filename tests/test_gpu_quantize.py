@@ -3,6 +3,7 @@ import numpy as np
 import pytest
 import torch
 
+from helpers import make_acts
 from oracle import uniql_oracle as orc
 
 pytestmark = pytest.mark.gpu
@@ -142,3 +143,24 @@ def test_rtn_without_reference_weights_on_any_bit_pattern(n_out, k_in):
     _, packed2, scales2 = ops.w4a16_quantize(w, want_ref=False)
     assert torch.equal(packed, packed2)
     assert torch.equal(scales.view(torch.int16), scales2.view(torch.int16))
+
+
+@pytest.mark.parametrize("rows", [1, 4, 8, 16, 64, 128, 200])
+def test_a_layer_runs_right_behind_the_kernel_that_packs_it(rows):
+    """from_fp16 and forward back to back on one stream, buffers freshly allocated and reused by the next layer: the linear
+    launches as a programmatic dependent and may not read weights or scales before the packing kernel has ended."""
+    from uniql_b200.quantize.quant_linear_layers import W4A16B16O16Linear
+    n, k = 4096, 4096
+    x = make_acts(rows, rows, k).cuda()
+    srcs = []
+    for i in range(4):
+        lin = torch.nn.Linear(k, n, bias=False, device="cuda", dtype=torch.float16)
+        lin.weight.data.normal_(0, 0.02)
+        srcs.append(lin)
+    settled = [W4A16B16O16Linear.from_fp16(lin) for lin in srcs]
+    torch.cuda.synchronize()
+    want = [mod(x) for mod in settled]
+    for _ in range(5):
+        got = [W4A16B16O16Linear.from_fp16(lin)(x) for lin in srcs]
+        for g, w in zip(got, want):
+            assert torch.equal(g, w)

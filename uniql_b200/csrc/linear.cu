@@ -57,7 +57,8 @@ static int check_proj(const uniql_w4a16_proj& q, int64_t k) {
   return UNIQL_OK;
 }
 
-static int group_launch(const CommView* cv, int64_t k_offset, const void* A, int64_t lda, int64_t m, int64_t k,
+// early_weights: the caller rules out that the kernel in front of this call in the stream wrote weights or scales.
+static int group_launch(const CommView* cv, bool early_weights, int64_t k_offset, const void* A, int64_t lda, int64_t m, int64_t k,
                         const uniql_w4a16_proj* proj, int nproj, int epilogue, const void* residual, int64_t ldr,
                         int64_t hadamard_dim, const uniql_prefetch* next, int nnext, void* scratch,
                         size_t scratch_bytes, int* status_word, cudaStream_t stream) {
@@ -82,6 +83,7 @@ static int group_launch(const CommView* cv, int64_t k_offset, const void* A, int
     if (!gemm_swap_supported(m, k, widths, nproj)) return UNIQL_ESHAPE;
     SwapArgs sa{};
     sa.projs = la; sa.Ds = ds; sa.nproj = nproj; sa.A = (const __half*)A; sa.lda = lda; sa.m = m;
+    sa.early_weights = early_weights;
     return launch_gemm_swap(sa, stream);
   }
   if (epilogue != UNIQL_EPILOGUE_NONE && epilogue != UNIQL_EPILOGUE_SWIGLU) return UNIQL_EINVAL;
@@ -121,6 +123,7 @@ static int group_launch(const CommView* cv, int64_t k_offset, const void* A, int
   a.scratch = scratch; a.scratch_bytes = scratch_bytes;
   a.status_word = status_word;
   a.comm = cv;
+  a.early_weights = early_weights;
   a.nprefetch = 0;
   if (next)
     for (int i = 0; i < nnext && a.nprefetch < UNIQL_MAX_PREFETCH; ++i)
@@ -176,7 +179,7 @@ extern "C" int uniql_w4a16_linear(const void* A, int64_t lda, const void* B, con
   uniql_w4a16_proj q;
   q.B = B; q.s = s; q.bias = bias; q.D = D; q.ldd = ldd; q.n = n; q.n_out = n_out;
   if (m <= 16)
-    return group_launch(nullptr, 0, A, lda, m, k, &q, 1, UNIQL_EPILOGUE_NONE, nullptr, 0, hadamard_dim, nullptr, 0,
+    return group_launch(nullptr, false, 0, A, lda, m, k, &q, 1, UNIQL_EPILOGUE_NONE, nullptr, 0, hadamard_dim, nullptr, 0,
                         scratch, scratch_bytes, status_word, stream);
 
   // m > 16: Hadamard (if any) as its own kernel into scratch, then the tensor-core kernels
@@ -196,13 +199,13 @@ extern "C" int uniql_w4a16_linear(const void* A, int64_t lda, const void* B, con
   if (tc) {
     LinearArgs a;
     a.B = B; a.s = s; a.bias = bias; a.ldd = ldd; a.n = n; a.n_out = n_out; a.k = k; a.status_word = status_word;
-    return launch_gemm_tc(a, Ain, lda, (__half*)D, m, stream);
+    return launch_gemm_tc(a, Ain, lda, (__half*)D, m, hadamard_dim != 0, stream);
   }
   const size_t slab_bytes = scratch_bytes - (hadamard_dim ? align_up((size_t)m * k * 2, 256) : 0);
   for (int64_t m0 = 0; m0 < m; m0 += 16) {
     const int64_t mc = m - m0 < 16 ? m - m0 : 16;
     q.D = (__half*)D + m0 * ldd;
-    int st = group_launch(nullptr, 0, Ain + m0 * lda, lda, mc, k, &q, 1, UNIQL_EPILOGUE_NONE, nullptr, 0, 0, nullptr, 0,
+    int st = group_launch(nullptr, false, 0, Ain + m0 * lda, lda, mc, k, &q, 1, UNIQL_EPILOGUE_NONE, nullptr, 0, 0, nullptr, 0,
                           scratch, slab_bytes, status_word, stream);
     if (st != UNIQL_OK) return st;
   }
@@ -213,15 +216,14 @@ extern "C" int uniql_w4a16_linear_group(const void* A, int64_t lda, int64_t m, i
                                         const uniql_w4a16_proj* proj, int nproj, int epilogue, const void* residual,
                                         int64_t ldr, int64_t hadamard_dim, const uniql_prefetch* next, int nnext,
                                         void* scratch, size_t scratch_bytes, int* status_word, void* stream) {
-  return uniql::group_launch(nullptr, 0, A, lda, m, k, proj, nproj, epilogue, residual, ldr, hadamard_dim, next, nnext,
+  return uniql::group_launch(nullptr, true, 0, A, lda, m, k, proj, nproj, epilogue, residual, ldr, hadamard_dim, next, nnext,
                              scratch, scratch_bytes, status_word, (cudaStream_t)stream);
 }
 
-extern "C" int uniql_w4a16_linear_group_tp(void* comm, int flags, int64_t col_offset, int64_t k_offset, const void* A,
-                                           int64_t lda, int64_t m, int64_t k, const uniql_w4a16_proj* proj, int nproj,
-                                           int epilogue, const void* residual, int64_t ldr, int64_t hadamard_dim,
-                                           const uniql_prefetch* next, int nnext, void* scratch,
-                                           size_t scratch_bytes, int* status_word, void* stream) {
+static int group_tp(void* comm, int flags, bool early_weights, int64_t col_offset, int64_t k_offset, const void* A, int64_t lda,
+                    int64_t m, int64_t k, const uniql_w4a16_proj* proj, int nproj, int epilogue, const void* residual,
+                    int64_t ldr, int64_t hadamard_dim, const uniql_prefetch* next, int nnext, void* scratch,
+                    size_t scratch_bytes, int* status_word, void* stream) {
   using namespace uniql;
   if (!comm || (flags & ~(UNIQL_TP_REDUCE | UNIQL_TP_GATHER_OUT | UNIQL_TP_GATHER_IN))) return UNIQL_EINVAL;
   if ((flags & UNIQL_TP_REDUCE) && (flags & UNIQL_TP_GATHER_OUT)) return UNIQL_EINVAL;
@@ -234,8 +236,17 @@ extern "C" int uniql_w4a16_linear_group_tp(void* comm, int flags, int64_t col_of
   cv.gather_out = (flags & UNIQL_TP_GATHER_OUT) ? 1 : 0;
   cv.gather_in = (flags & UNIQL_TP_GATHER_IN) ? 1 : 0;
   cv.col_offset = col_offset;
-  return group_launch(&cv, k_offset, A, lda, m, k, proj, nproj, epilogue, residual, ldr, hadamard_dim, next, nnext,
+  return group_launch(&cv, early_weights, k_offset, A, lda, m, k, proj, nproj, epilogue, residual, ldr, hadamard_dim, next, nnext,
                       scratch, scratch_bytes, status_word, (cudaStream_t)stream);
+}
+
+extern "C" int uniql_w4a16_linear_group_tp(void* comm, int flags, int64_t col_offset, int64_t k_offset, const void* A,
+                                           int64_t lda, int64_t m, int64_t k, const uniql_w4a16_proj* proj, int nproj,
+                                           int epilogue, const void* residual, int64_t ldr, int64_t hadamard_dim,
+                                           const uniql_prefetch* next, int nnext, void* scratch,
+                                           size_t scratch_bytes, int* status_word, void* stream) {
+  return group_tp(comm, flags, true, col_offset, k_offset, A, lda, m, k, proj, nproj, epilogue, residual, ldr, hadamard_dim,
+                  next, nnext, scratch, scratch_bytes, status_word, stream);
 }
 
 extern "C" int uniql_w4a16_linear_allreduce(void* comm, const void* A, int64_t lda, const void* B, const void* s,
@@ -246,8 +257,8 @@ extern "C" int uniql_w4a16_linear_allreduce(void* comm, const void* A, int64_t l
   if (n_out <= 0 || n_out > n) return UNIQL_EINVAL;
   uniql_w4a16_proj q;
   q.B = B; q.s = s; q.bias = bias; q.D = D; q.ldd = ldd; q.n = n; q.n_out = n_out;
-  return uniql_w4a16_linear_group_tp(comm, UNIQL_TP_REDUCE, 0, 0, A, lda, m, k, &q, 1, UNIQL_EPILOGUE_NONE, nullptr, 0,
-                                     0, nullptr, 0, scratch, scratch_bytes, status_word, stream);
+  return group_tp(comm, UNIQL_TP_REDUCE, false, 0, 0, A, lda, m, k, &q, 1, UNIQL_EPILOGUE_NONE, nullptr, 0, 0, nullptr, 0,
+                  scratch, scratch_bytes, status_word, stream);
 }
 
 extern "C" int uniql_abi_version(void) { return UNIQL_ABI_VERSION; }

@@ -53,6 +53,7 @@ struct DecodeArgs {
   size_t scratch_bytes;
   int* status_word;
   const CommView* comm;       // nullptr: single GPU
+  bool early_weights;         // the launch may fetch weights and scales before its predecessor in the stream has ended
   int nprefetch;              // byte ranges to pull into L2 as the launch ends (weights of the launches that follow)
   const void* prefetch_ptr[4];
   size_t prefetch_bytes[4];
@@ -60,7 +61,7 @@ struct DecodeArgs {
 
 // CTA-tiled decode kernel (w4a16_gemv.cu): single-GPU launches, activations already transformed.
 size_t gemv_scratch_bytes(int64_t m, int64_t k, const int64_t* n, int nproj, int epilogue);
-int launch_gemv_group(const DecodeArgs& a, const __half* A, int64_t lda, cudaStream_t stream);
+int launch_gemv_group(const DecodeArgs& a, const __half* A, int64_t lda, bool early_weights, cudaStream_t stream);
 
 // m <= 16.  Scratch bytes the launch needs (tickets included).
 size_t decode_scratch_bytes(int64_t m, int64_t k, const int64_t* n, int nproj, int epilogue, int64_t hadamard_dim,
@@ -79,7 +80,7 @@ struct LinearArgs {
 // Tensor-core (tcgen05) path for m > 16.
 bool gemm_tc_supported(int64_t m, int64_t n, int64_t k);
 size_t gemm_tc_scratch_bytes(int64_t m, int64_t n, int64_t k);
-int launch_gemm_tc(const LinearArgs& a, const __half* A, int64_t lda, __half* D, int64_t m, cudaStream_t stream);
+int launch_gemm_tc(const LinearArgs& a, const __half* A, int64_t lda, __half* D, int64_t m, bool early_weights, cudaStream_t stream);
 // Operand-swapped tensor-core kernel (w4a16_gemm_swap.cu): up to kMaxProj projections that read the same activations
 // (same k) as one launch; Ds[i] receives projection i (leading dimension projs[i].ldd).
 struct SwapArgs {
@@ -91,6 +92,7 @@ struct SwapArgs {
   int64_t ldr;
   const __half* A;
   int64_t lda, m;
+  bool early_weights;         // as in DecodeArgs
   const CommView* comm;       // at most 16 rows: the exchanges of a tensor-parallel step; nullptr: single GPU
 };
 bool gemm_swap_supported(int64_t m, int64_t k, const int64_t* n, int nproj);

@@ -31,8 +31,8 @@
 // clears them, and applies the epilogue: bias, SwiGLU product of a gate/up pair, residual add, fp16 store.  For up to
 // four rows the online Hadamard transform of the activations runs in the kernel's own prologue.
 //
-// Every launch carries the programmatic-dependent-launch attribute, fills its rings, releases its own dependents and only
-// then waits for its predecessor.  Measured against the tiled kernel this kernel is slower (its reduction crosses global
+// Where the predecessor cannot have written the weights, a launch carries the programmatic-dependent-launch attribute, fills
+// its rings, releases its own dependents and only then waits for its predecessor.  Measured against the tiled kernel this kernel is slower (its reduction crosses global
 // memory); it is kept as a tested alternative.
 //
 // Roofline: HBM.  Algorithmic bytes per launch = sum over projections of k*n/2 + (k/128)*n*2 + m*n_out*2, + m*k*2.
@@ -1049,7 +1049,7 @@ static bool use_slot_engine(const DecodeArgs& a) {
 }
 
 template <int MT, int WARPS, int MINB, bool HAD, int RING>
-static int launch_variant(const DecodeParams& p, const DecodePlan& pl, cudaStream_t stream) {
+static int launch_variant(const DecodeParams& p, const DecodePlan& pl, bool pdl, cudaStream_t stream) {
   auto kern = w4a16_decode_kernel<MT, WARPS, MINB, HAD, RING>;
   {
     // function attributes are per device; raise the dynamic shared-memory limit to what this launch needs
@@ -1069,10 +1069,10 @@ static int launch_variant(const DecodeParams& p, const DecodePlan& pl, cudaStrea
   cfg.stream = stream;
   cudaLaunchAttribute attr[1];
   int nattr = 0;
-  // Every launch may start early behind its predecessor; the kernel itself waits (griddepcontrol.wait)
-  // before it touches anything another kernel could have written.
+  // The launch may start early behind its predecessor where that cannot have written the weights; the kernel itself waits
+  // (griddepcontrol.wait) before it touches anything else another kernel could have written.
   static const int pdl_on = env_int("UNIQL_B200_PDL", 1);
-  if (pdl_on) {
+  if (pdl_on && pdl) {
     attr[nattr].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[nattr].val.programmaticStreamSerializationAllowed = 1;
     ++nattr;
@@ -1131,6 +1131,8 @@ int launch_decode(const DecodeArgs& a, cudaStream_t stream) {
       if (st != UNIQL_OK) return st;
       lda = a.hadamard_dim;
     }
+    // the transform is a launch of its own that starts when everything in front of it has ended
+    const bool early_weights = a.early_weights || a.hadamard_dim != 0;
     // From five rows on, with and without a communicator (a step of a tensor-parallel layer has the sums of the plain
     // launch), the tensor-core kernel with exact codes as the operand and fp32 group scales (the arithmetic of the
     // tiled kernel) is faster: its work per weight does not grow with the rows, while the tiled kernel stages rows x k
@@ -1149,9 +1151,10 @@ int launch_decode(const DecodeArgs& a, cudaStream_t stream) {
       sa.projs = la; sa.Ds = ds; sa.nproj = a.nproj; sa.pair = a.epilogue == UNIQL_EPILOGUE_SWIGLU;
       sa.residual = a.residual; sa.ldr = a.ldr; sa.A = Ain; sa.lda = lda; sa.m = a.m;
       sa.comm = a.comm;
+      sa.early_weights = early_weights;
       return launch_gemm_swap(sa, stream);
     }
-    return launch_gemv_group(a, Ain, lda, stream);
+    return launch_gemv_group(a, Ain, lda, early_weights, stream);
   }
   DecodePlan pl;
   int st = cached_plan(&pl, a.m, a.k, n, a.nproj, a.epilogue, a.hadamard_dim, a.k_offset);
@@ -1215,14 +1218,14 @@ int launch_decode(const DecodeArgs& a, cudaStream_t stream) {
       ++p.npf;
     }
   if (pl.fused_had) {
-    if (pl.variant == 0) return launch_variant<1, 16, 1, true, 3>(p, pl, stream);
-    if (pl.variant == 3) return launch_variant<1, 8, 2, true, 2>(p, pl, stream);
-    return launch_variant<1, 16, 1, true, 2>(p, pl, stream);     // m <= 4 here
+    if (pl.variant == 0) return launch_variant<1, 16, 1, true, 3>(p, pl, a.early_weights, stream);
+    if (pl.variant == 3) return launch_variant<1, 8, 2, true, 2>(p, pl, a.early_weights, stream);
+    return launch_variant<1, 16, 1, true, 2>(p, pl, a.early_weights, stream);     // m <= 4 here
   }
-  if (pl.variant == 0) return launch_variant<1, 16, 1, false, 3>(p, pl, stream);
-  if (pl.variant == 1) return launch_variant<1, 16, 1, false, 2>(p, pl, stream);
-  if (pl.variant == 3) return launch_variant<1, 8, 2, false, 2>(p, pl, stream);
-  return launch_variant<2, 12, 1, false, 2>(p, pl, stream);
+  if (pl.variant == 0) return launch_variant<1, 16, 1, false, 3>(p, pl, a.early_weights, stream);
+  if (pl.variant == 1) return launch_variant<1, 16, 1, false, 2>(p, pl, a.early_weights, stream);
+  if (pl.variant == 3) return launch_variant<1, 8, 2, false, 2>(p, pl, a.early_weights, stream);
+  return launch_variant<2, 12, 1, false, 2>(p, pl, a.early_weights, stream);
 }
 
 // Host-side replay of the kernel's work split for one launch geometry: walks every warp's slots with the kernel's own

@@ -92,6 +92,7 @@ struct SwapParams {
   int nissue;                                   // issuing threads (1 or 2; with 2, nst is even: a stage has one issuer)
   int nbuf;                                     // tiles whose accumulators are kept (1 or 2)
   int off_x;                                    // activation ring in shared memory
+  int early_weights;                            // 0: weights and scales may have been written by the preceding kernel
   int* status_word;
   CommView cv;                                  // tensor-parallel launches only
 };
@@ -281,7 +282,9 @@ w4a16_gemm_swap_kernel(const __grid_constant__ SwapParams p, const __grid_consta
   const int total_it = my_tiles * KB;
   const int tmem_w0 = TMEM_COLS - p.nst * (BK / 2);   // weight tile of stage s: columns tmem_w0 + 64 s
 
-  pdl_launch_dependents();                       // the next kernel in the stream may start its own set-up and weights
+  // the next kernel in the stream may start its own set-up and weights; where this launch waits for its predecessor first,
+  // behind that wait, so that what starts behind this launch may rely on the predecessor too
+  if (p.early_weights) pdl_launch_dependents();
   // Packed words of k-block kb of column tile (pi, lt): two boxes, one barrier.
   auto load_packed = [&](int pi, int lt, int kb, int sp) {
     const int x0 = PAIR ? lt * 128 : lt * 256;
@@ -302,6 +305,7 @@ w4a16_gemm_swap_kernel(const __grid_constant__ SwapParams p, const __grid_consta
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     int pi, lt;
     sw_tile_of(p, tile0 / p.rtiles, pi, lt);
+    if (!p.early_weights) pdl_wait();
     for (int kb = 0; kb < early; ++kb) load_packed(pi, lt, kb, kb);
   }
   if (warp == 2 && tc_elect()) {
@@ -329,6 +333,10 @@ w4a16_gemm_swap_kernel(const __grid_constant__ SwapParams p, const __grid_consta
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
   bool timed_out = false;
+  if (!p.early_weights) {
+    pdl_wait();                                  // before the first scale is read
+    pdl_launch_dependents();
+  }
 
   // TP: finishes rows [r0, r1) of a tile with `nthreads` threads, four columns of a row per thread and step; `quad` delivers
   // the sums of four adjacent columns of the tile.  kQuads divides every nthreads, so a thread stays in one 64-column block.
@@ -974,6 +982,7 @@ int launch_gemm_swap(const SwapArgs& a, cudaStream_t stream) {
   p.rtiles = shape.rtiles;
   p.ntiles = ctiles * p.rtiles;
   p.status_word = a.projs[0].status_word;
+  p.early_weights = a.early_weights ? 1 : 0;
   CUtensorMap xmap;
   {
     // [k / 64][rows][64 k]: one box brings both swizzled 64-k sub-tiles of a stage
@@ -998,8 +1007,8 @@ int launch_gemm_swap(const SwapArgs& a, cudaStream_t stream) {
   cfg.stream = stream;
   cudaLaunchAttribute attr[2];
   int nattr = 0;
-  // May start behind its predecessor; the kernel waits (griddepcontrol.wait) before it reads the activations, but not for
-  // the weights and scales: callers of the entry points above 128 rows may have written those just before.
+  // May start behind its predecessor; the kernel waits (griddepcontrol.wait) before it reads the activations, and before it
+  // reads weights and scales too unless the caller rules out that the predecessor wrote them.
   static const int pdl_on = swap_env("UNIQL_B200_PDL", 1);
   if (pdl_on && m <= 128) {
     attr[nattr].id = cudaLaunchAttributeProgrammaticStreamSerialization;

@@ -368,12 +368,13 @@ static bool prefill_tiles_win(int64_t m, int64_t n, int64_t k) {
   return cycles < 1.12 * gemm_swap_cycles(m, k, (int)((n + 127) / 128));
 }
 
-int launch_gemm_tc(const LinearArgs& a, const __half* A, int64_t lda, __half* D, int64_t m, cudaStream_t stream) {
+int launch_gemm_tc(const LinearArgs& a, const __half* A, int64_t lda, __half* D, int64_t m, bool early_weights, cudaStream_t stream) {
   using namespace tc;
   if (!prefill_tiles_win(m, a.n, a.k)) {
     void* d1[1] = {D};
     SwapArgs sa{};
     sa.projs = &a; sa.Ds = d1; sa.nproj = 1; sa.A = A; sa.lda = lda; sa.m = m;
+    sa.early_weights = early_weights;
     return launch_gemm_swap(sa, stream);
   }
   EncodeTiledFn enc = encode_tiled_fn();

@@ -20,8 +20,8 @@
 // memory in a fixed order; CTAs along k (S <= 8) form a thread-block cluster and add up their tiles through
 // distributed shared memory, for S > 8 they write fp32 partials to scratch and the last one to arrive (atomic ticket,
 // no spinning) adds them in a fixed order -> deterministic results, no inter-CTA waits outside a cluster barrier.
-// Every launch is a programmatic dependent: it starts its weight stream, releases its own dependents and only then
-// waits for the producer of its activations.
+// Every launch is a programmatic dependent: where the caller rules out that the preceding kernel wrote the weights it starts
+// its weight stream, releases its own dependents and only then waits for the producer of its activations.
 //
 // Grouped launches.  Up to four projections that read the same activations form one launch: their 64-column blocks
 // are laid side by side in one virtual column space (block by block for q/k/v; gate and up blocks interleaved for a
@@ -87,6 +87,7 @@ struct GemvParams {
   const unsigned char* pf_ptr[4];   // byte ranges to pull into L2 when this launch's weight stream ends
   long long pf_lines[4];
   int npf;
+  int early_weights;    // 0: wait for the preceding kernel before the first weight load (it may have written them)
   CommView cv;          // tensor parallelism: cross-GPU sum of a row-parallel shard / feature gather of a column shard
 };
 
@@ -250,6 +251,7 @@ w4a16_gemv_kernel(const __grid_constant__ GemvParams p) {
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
   }
   __syncwarp();
+  if (!p.early_weights) pdl_wait();    // ahead of the release below: what starts behind this launch may rely on it
   // ---- start streaming weights before anything else: one TMA tile per group and 64-column block ----
   if (has_work && lane == 0) {
     for (int s = 0; s < p.R; ++s)
@@ -809,7 +811,7 @@ size_t gemv_scratch_bytes(int64_t m, int64_t k, const int64_t* n, int nproj, int
 }
 
 // A: the activations the kernel multiplies with (already transformed if the layer has an online Hadamard).
-int launch_gemv_group(const DecodeArgs& a, const __half* A, int64_t lda, cudaStream_t stream) {
+int launch_gemv_group(const DecodeArgs& a, const __half* A, int64_t lda, bool early_weights, cudaStream_t stream) {
   if (a.nproj < 1 || a.nproj > kMaxProj || a.m < 1 || a.m > 16 || a.k % 128) return UNIQL_ESHAPE;
   const bool pair = a.epilogue == UNIQL_EPILOGUE_SWIGLU;
   if (pair && (a.nproj != 2 || a.proj[0].n != a.proj[1].n)) return UNIQL_EINVAL;
@@ -852,6 +854,7 @@ int launch_gemv_group(const DecodeArgs& a, const __half* A, int64_t lda, cudaStr
   const int grid_x = (p.nblk + p.WN - 1) / p.WN;
   if ((size_t)grid_x * sizeof(int) > UNIQL_SCRATCH_COUNTER_BYTES) return UNIQL_ESHAPE;
   if (a.comm) p.cv = *a.comm;
+  p.early_weights = early_weights ? 1 : 0;
   p.npf = 0;
   for (int i = 0; i < a.nprefetch && i < 4; ++i)
     if (a.prefetch_ptr[i] && a.prefetch_bytes[i] >= 128) {
@@ -880,8 +883,8 @@ int launch_gemv_group(const DecodeArgs& a, const __half* A, int64_t lda, cudaStr
   cfg.stream = stream;
   cudaLaunchAttribute attr[2];
   int nattr = 0;
-  // Every launch may start early behind its predecessor; the kernel itself waits (griddepcontrol.wait)
-  // before it touches anything another kernel could have written.
+  // Every launch may start early behind its predecessor; the kernel itself waits (griddepcontrol.wait) before it touches
+  // anything another kernel could have written: weights and scales too, unless the caller rules that out.
   static const int pdl_on = env_int("UNIQL_B200_PDL", 1);
   if (pdl_on) {
     attr[nattr].id = cudaLaunchAttributeProgrammaticStreamSerialization;
