@@ -91,3 +91,20 @@ def test_packed_ring_refilled_many_times(m):
     _check(first, x, layer)
     for _ in range(20):
         assert torch.equal(ops.w4a16_linear(x.cuda(), w, s, b, n), first)
+
+
+@pytest.mark.parametrize("m", [1, 5, 16, 17, 128])
+def test_prefetch_hint(m):
+    """The ranges are asked for by every grouped launch, whole 128-byte lines inside them only, and change no result.
+    (Lines are dealt out over CTAs and lanes: no line, one, fewer than lanes, many.)"""
+    from uniql_b200 import ops
+    n, k = 1024, 1024
+    layer = quantized_layer(n + k, n, k)
+    x = make_acts(m, m, k).cuda()
+    hints = [(torch.zeros(nb, dtype=torch.uint8, device="cuda"), nb) for nb in (100, 128, 3000, 1 << 22)]
+    (want,) = ops.w4a16_linear_group(x, [_dev(layer)])
+    (got,) = ops.w4a16_linear_group(x, [_dev(layer)], prefetch=hints)
+    torch.cuda.synchronize()
+    assert torch.equal(got, want)
+    _check(got, x.cpu(), layer)
+    assert ops.read_and_clear_status("cuda") == 0

@@ -64,6 +64,16 @@ static int group_launch(const CommView* cv, bool early_weights, int64_t k_offset
                         size_t scratch_bytes, int* status_word, cudaStream_t stream) {
   if (!proj || nproj < 1 || nproj > UNIQL_MAX_PROJ || m < 0 || k <= 0) return UNIQL_EINVAL;
   if (k % 128 != 0) return UNIQL_ESHAPE;
+  int npf = 0;
+  const void* pf_ptr[UNIQL_MAX_PREFETCH];
+  size_t pf_bytes[UNIQL_MAX_PREFETCH];
+  if (next)
+    for (int i = 0; i < nnext && npf < UNIQL_MAX_PREFETCH; ++i)
+      if (next[i].ptr && next[i].bytes) {
+        pf_ptr[npf] = next[i].ptr;
+        pf_bytes[npf] = next[i].bytes;
+        ++npf;
+      }
   if (m > 16) {
     // 17..128 rows: the projections share one launch of the operand-swapped tensor-core kernel (plain outputs only:
     // the elementwise epilogues, the transform and the tensor-parallel exchanges belong to the decode kernel)
@@ -84,6 +94,7 @@ static int group_launch(const CommView* cv, bool early_weights, int64_t k_offset
     SwapArgs sa{};
     sa.projs = la; sa.Ds = ds; sa.nproj = nproj; sa.A = (const __half*)A; sa.lda = lda; sa.m = m;
     sa.early_weights = early_weights;
+    sa.nprefetch = npf; sa.prefetch_ptr = pf_ptr; sa.prefetch_bytes = pf_bytes;
     return launch_gemm_swap(sa, stream);
   }
   if (epilogue != UNIQL_EPILOGUE_NONE && epilogue != UNIQL_EPILOGUE_SWIGLU) return UNIQL_EINVAL;
@@ -124,14 +135,8 @@ static int group_launch(const CommView* cv, bool early_weights, int64_t k_offset
   a.status_word = status_word;
   a.comm = cv;
   a.early_weights = early_weights;
-  a.nprefetch = 0;
-  if (next)
-    for (int i = 0; i < nnext && a.nprefetch < UNIQL_MAX_PREFETCH; ++i)
-      if (next[i].ptr && next[i].bytes) {
-        a.prefetch_ptr[a.nprefetch] = next[i].ptr;
-        a.prefetch_bytes[a.nprefetch] = next[i].bytes;
-        ++a.nprefetch;
-      }
+  a.nprefetch = npf;
+  for (int i = 0; i < npf; ++i) { a.prefetch_ptr[i] = pf_ptr[i]; a.prefetch_bytes[i] = pf_bytes[i]; }
   return launch_decode(a, stream);
 }
 

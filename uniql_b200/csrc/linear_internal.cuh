@@ -93,6 +93,9 @@ struct SwapArgs {
   const __half* A;
   int64_t lda, m;
   bool early_weights;         // as in DecodeArgs
+  int nprefetch;              // as in DecodeArgs
+  const void* const* prefetch_ptr;
+  const size_t* prefetch_bytes;
   const CommView* comm;       // at most 16 rows: the exchanges of a tensor-parallel step; nullptr: single GPU
 };
 bool gemm_swap_supported(int64_t m, int64_t k, const int64_t* n, int nproj);

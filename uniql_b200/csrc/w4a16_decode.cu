@@ -1152,6 +1152,7 @@ int launch_decode(const DecodeArgs& a, cudaStream_t stream) {
       sa.residual = a.residual; sa.ldr = a.ldr; sa.A = Ain; sa.lda = lda; sa.m = a.m;
       sa.comm = a.comm;
       sa.early_weights = early_weights;
+      sa.nprefetch = a.nprefetch; sa.prefetch_ptr = a.prefetch_ptr; sa.prefetch_bytes = a.prefetch_bytes;
       return launch_gemm_swap(sa, stream);
     }
     return launch_gemv_group(a, Ain, lda, early_weights, stream);

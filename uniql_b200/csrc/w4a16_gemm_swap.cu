@@ -92,6 +92,9 @@ struct SwapParams {
   int nissue;                                   // issuing threads (1 or 2; with 2, nst is even: a stage has one issuer)
   int nbuf;                                     // tiles whose accumulators are kept (1 or 2)
   int off_x;                                    // activation ring in shared memory
+  const unsigned char* pf_ptr[4];               // byte ranges to pull into L2 when this CTA's weight stream ends, in
+  long long pf_lines[4];                        // 128-byte lines
+  int npf;
   int early_weights;                            // 0: weights and scales may have been written by the preceding kernel
   int* status_word;
   CommView cv;                                  // tensor-parallel launches only
@@ -456,6 +459,12 @@ w4a16_gemm_swap_kernel(const __grid_constant__ SwapParams p, const __grid_consta
         }
       }
     }
+    // The last packed words are on their way: ask L2 for this CTA's share of the weights that the following launches will
+    // stream, so that HBM keeps working while this launch converts, reduces and drains (plain per-line hints).
+    __syncwarp();
+    for (int r = 0; r < p.npf; ++r)
+      for (long long l = (long long)blockIdx.x * 32 + lane; l < p.pf_lines[r]; l += (long long)gridDim.x * 32)
+        asm volatile("prefetch.global.L2 [%0];" ::"l"(p.pf_ptr[r] + l * 128));
   } else if (warp == 2) {
     // ------------------------------------------------------------------ activation producer (re-reads, L2 hits)
     if (tc_elect()) {
@@ -983,6 +992,12 @@ int launch_gemm_swap(const SwapArgs& a, cudaStream_t stream) {
   p.ntiles = ctiles * p.rtiles;
   p.status_word = a.projs[0].status_word;
   p.early_weights = a.early_weights ? 1 : 0;
+  for (int i = 0; i < a.nprefetch && i < 4; ++i)
+    if (a.prefetch_ptr[i] && a.prefetch_bytes[i] >= 128) {
+      p.pf_ptr[p.npf] = (const unsigned char*)a.prefetch_ptr[i];
+      p.pf_lines[p.npf] = (long long)(a.prefetch_bytes[i] / 128);
+      ++p.npf;
+    }
   CUtensorMap xmap;
   {
     // [k / 64][rows][64 k]: one box brings both swizzled 64-k sub-tiles of a stage
