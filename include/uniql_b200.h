@@ -323,8 +323,9 @@ int uniql_w4a16_plan_selftest(int64_t m, int64_t k, const int64_t* n, int nproj,
 int uniql_w4a16_gemv_plan_check(int64_t m, int64_t k, const int64_t* n, int nproj, int epilogue, int64_t* out5);
 
 /* Host-only check of every plan the operand-swapped tensor-core kernel can be launched with (ring depths against the
- * number of dequantise sets and issuing threads, tensor-memory columns, shared memory).  Returns 0, or the row-tile size
- * whose plan breaks a rule the kernel relies on. */
+ * number of dequantise sets and issuing threads, tensor-memory columns, shared memory), and that every launch gets row tiles
+ * and a k-split, also when UNIQL_B200_TC_SPLIT asks for one that is too large.  Returns 0, or the row-tile size whose plan
+ * breaks a rule the kernel relies on, or 1000 + the scale groups of a launch that gets no shape. */
 int uniql_w4a16_swap_plan_check(void);
 
 #ifdef __cplusplus

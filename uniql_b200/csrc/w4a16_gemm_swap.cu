@@ -885,15 +885,20 @@ static bool swap_plan_ok(const SwapPlan& pl, int Mb, bool gs) {
 // epilogue has no second accumulator to hide behind adds ~20 cycles a row; a cluster sum ~3000.  14336 x 4096, 160 rows:
 // 628 cycles a stage measured (640 by the pipe), 224 rows 865 (896); above 224 rows the activation ring has room for two
 // stages only: 256 rows 1153 (1024).
+static int swap_forced_split() {
+  static const int forced = swap_env("UNIQL_B200_TC_SPLIT", 0);
+  return forced;
+}
 struct SwapShape {
   int rtiles, Mb, split;
   double cycles;
 };
-static SwapShape swap_shape(int64_t m, int64_t k, int ctiles, bool gs) {
+// forced > 0: that k-split instead (the largest possible one where it is too large), for tests and profiling.
+static SwapShape swap_shape(int64_t m, int64_t k, int ctiles, bool gs, int forced) {
   using namespace sw;
-  static const int forced = swap_env("UNIQL_B200_TC_SPLIT", 0);
   const int sms = device_info().sm_count;
   const int groups = (int)(k / 128);
+  forced = min(forced, min(8, groups));
   SwapShape best{};
   best.cycles = 1e30;
   const int rt0 = (int)((m + MB_MAX - 1) / MB_MAX), rt1 = m <= 128 ? 1 : rt0 + 2;
@@ -903,7 +908,7 @@ static SwapShape swap_shape(int64_t m, int64_t k, int ctiles, bool gs) {
     const int64_t tiles = (int64_t)ctiles * rt;
     const double stage = Mb > 224 ? 4.5 * Mb : Mb > 107 ? 4.0 * Mb : 430.0;
     for (int split = 1; split <= 8; ++split) {
-      if (forced > 0 ? split != (forced > groups ? groups : forced) : (split > 1 && (tiles * split > sms || groups / split < 4)))
+      if (forced > 0 ? split != forced : (split > 1 && (tiles * split > sms || groups / split < 4)))
         continue;
       // every cluster must be resident at once (a second wave would cost more than the split gains): clusters are placed
       // inside one GPC, so fewer fit than SMs / split suggests
@@ -923,7 +928,7 @@ static SwapShape swap_shape(int64_t m, int64_t k, int ctiles, bool gs) {
 static int swap_set_attributes(bool gs, bool pair, bool tp);
 double gemm_swap_cycles(int64_t m, int64_t k, int ctiles) {
   if (swap_set_attributes(m <= 16, false, false) != UNIQL_OK) return 1e30;
-  return swap_shape(m, k, ctiles, m <= 16).cycles;
+  return swap_shape(m, k, ctiles, m <= 16, swap_forced_split()).cycles;
 }
 
 bool gemm_swap_supported(int64_t m, int64_t k, const int64_t* n, int nproj) {
@@ -985,7 +990,8 @@ int launch_gemm_swap(const SwapArgs& a, cudaStream_t stream) {
     const int st = swap_set_attributes(gs, a.pair, a.comm != nullptr);
     if (st != UNIQL_OK) return st;
   }
-  const SwapShape shape = swap_shape(m, k, ctiles, gs);
+  const SwapShape shape = swap_shape(m, k, ctiles, gs, swap_forced_split());
+  if (shape.split < 1) return UNIQL_ESHAPE;
   const int Mb = shape.Mb, split = shape.split, sms = device_info().sm_count;
   p.M = (int)m; p.Mb = Mb; p.K = (int)k;
   p.rtiles = shape.rtiles;
@@ -1046,12 +1052,21 @@ int launch_gemm_swap(const SwapArgs& a, cudaStream_t stream) {
 }  // namespace uniql
 
 // Host-only check (no device work): every row tile this kernel can be launched with gets a plan that its barriers, tensor
-// memory and shared memory can hold.  0, or the row-tile size whose plan fails.
+// memory and shared memory can hold, and every launch gets row tiles that cover its rows and a k-split, whatever split is
+// asked for.  0, or the row-tile size whose plan fails, or 1000 + the scale groups of a launch without a shape.
 extern "C" int uniql_w4a16_swap_plan_check(void) {
   for (int Mb = 16; Mb <= uniql::sw::MB_MAX; Mb += 16)
     for (int one = 0; one < 2; ++one)
       for (int gs = 0; gs <= (Mb == 16 ? 1 : 0); ++gs)
         for (int kb = 1; kb <= 2; ++kb)
           if (!uniql::swap_plan_ok(uniql::swap_plan(Mb, gs != 0, one != 0, kb), Mb, gs != 0)) return Mb;
+  for (int groups : {1, 2, 3, 8, 9, 112})
+    for (int m : {5, 64, 256, 257, 4096})
+      for (int forced : {0, 1, 3, 8, 9, 64}) {
+        const uniql::SwapShape sh = uniql::swap_shape(m, (int64_t)groups * 128, 8, m <= 16, forced);
+        const bool covers = sh.Mb >= 16 && sh.Mb <= uniql::sw::MB_MAX && sh.Mb % 16 == 0 &&
+                            (int64_t)sh.rtiles * sh.Mb >= m && (int64_t)(sh.rtiles - 1) * sh.Mb < m;
+        if (!covers || sh.split < 1 || sh.split > 8 || sh.split > groups) return 1000 + groups;
+      }
   return 0;
 }
