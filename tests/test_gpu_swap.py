@@ -108,3 +108,34 @@ def test_prefetch_hint(m):
     assert torch.equal(got, want)
     _check(got, x.cpu(), layer)
     assert ops.read_and_clear_status("cuda") == 0
+
+
+@pytest.mark.parametrize("m", [5, 8, 16])
+@pytest.mark.parametrize("n,k", [(64, 1024), (200, 2304), (2048, 2048), (1024, 4096)])
+def test_swiglu_pair_and_residual_shared_by_a_cluster(m, n, k):
+    """1 to 32 pair tiles, so that a cluster shares each over k and the epilogue works on sums fetched from its CTAs' shared
+    memory.  Bounds: gate and up as in _check (ends in fp16 roundings of their own: included); |silu'| < 1.1; then the fp16
+    roundings of silu, product and sum, half an ulp = 2^-11 each, 2^-25 where the result is subnormal."""
+    from uniql_b200 import ops
+    gl, ul = (quantized_layer(i + n + k, n, k, bias=(n == 200)) for i in (1, 2))
+    x = make_acts(m, m, k)
+    res = make_acts(m + 1, m, n, outliers=False)
+
+    def parts(layer):
+        ref = orc.linear_ref(x.numpy(), None, None, layer["bias"], n, w_deq=layer["w_deq"]).astype(np.float64)
+        mass = np.abs(x.numpy().astype(np.float64)) @ np.abs(layer["w_deq"][:, :n].astype(np.float64))
+        return ref, 2.0 ** -10 * np.abs(ref) + (2 * layer["k"] * 2.0 ** -24 + 2.0 ** -11) * mass + 1e-7
+
+    (g, eg), (u, eu) = parts(gl), parts(ul)
+    act = g / (1.0 + np.exp(-g))
+    want = act * u
+    bound = 1.1 * eg * (np.abs(u) + eu) + np.abs(act) * eu
+    bound = bound + 2.0 ** -11 * (np.abs(act) + 1.1 * eg) * (np.abs(u) + eu) + 2.0 ** -25 * (np.abs(u) + eu)
+    bound = bound + 2.0 ** -11 * (np.abs(want) + bound) + 2.0 ** -24
+    for _ in range(3):
+        (got,) = ops.w4a16_linear_group(x.cuda(), [_dev(gl), _dev(ul)], epilogue="swiglu")
+        assert (np.abs(got.cpu().numpy().astype(np.float64) - want) <= bound).all()
+        (got,) = ops.w4a16_linear_group(x.cuda(), [_dev(gl)], residual=res.cuda())
+        summed = g + res.numpy().astype(np.float64)
+        assert (np.abs(got.cpu().numpy().astype(np.float64) - summed) <= eg + 2.0 ** -11 * (np.abs(summed) + eg) + 1e-7).all()
+    assert ops.read_and_clear_status("cuda") == 0
