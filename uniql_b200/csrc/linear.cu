@@ -33,8 +33,7 @@ static bool use_tc(int64_t m, int64_t n, int64_t k) { return m > 16 && gemm_tc_s
 // Hadamard in front) the transformed activations.
 static size_t linear_scratch_bytes(int64_t m, int64_t n, int64_t k, int64_t hadamard_dim) {
   if (use_tc(m, n, k))
-    return UNIQL_SCRATCH_COUNTER_BYTES + (hadamard_dim ? align_up((size_t)m * k * 2, 256) : 0) +
-           align_up(gemm_tc_scratch_bytes(m, n, k), 256);
+    return UNIQL_SCRATCH_COUNTER_BYTES + (hadamard_dim ? align_up((size_t)m * k * 2, 256) : 0);
   // decode kernel, in slabs of 16 rows when m > 16 (shapes the tensor-core kernels do not take)
   size_t need = decode_scratch_bytes(m > 16 ? 16 : m, k, &n, 1, UNIQL_EPILOGUE_NONE, m > 16 ? 0 : hadamard_dim, 0);
   if (m > 16) {

@@ -79,7 +79,6 @@ struct LinearArgs {
 
 // Tensor-core (tcgen05) path for m > 16.
 bool gemm_tc_supported(int64_t m, int64_t n, int64_t k);
-size_t gemm_tc_scratch_bytes(int64_t m, int64_t n, int64_t k);
 int launch_gemm_tc(const LinearArgs& a, const __half* A, int64_t lda, __half* D, int64_t m, bool early_weights, cudaStream_t stream);
 // Operand-swapped tensor-core kernel (w4a16_gemm_swap.cu): up to kMaxProj projections that read the same activations
 // (same k) as one launch; Ds[i] receives projection i (leading dimension projs[i].ldd).

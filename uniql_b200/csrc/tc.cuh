@@ -63,15 +63,6 @@ __device__ __forceinline__ uint64_t tc_smem_desc(uint32_t addr) {
   // K-major, 128-byte swizzle: 8-row groups 1024 bytes apart; descriptor version 1 (sm_100)
   return (uint64_t)((addr & 0x3FFFFu) >> 4) | (1ull << 16) | (64ull << 32) | (1ull << 46) | (2ull << 61);
 }
-__device__ __forceinline__ void tc_mma_f16(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc,
-                                           uint32_t accumulate) {
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
-      ::"r"(tmem_d), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
-      : "memory");
-}
 __device__ __forceinline__ void tc_commit(uint32_t bar) {
   asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
 }
@@ -86,22 +77,6 @@ __device__ __forceinline__ uint4 tc_lds128(uint32_t addr) {
   asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(addr) : "memory");
   return v;
 }
-// Wait used by warps that sit idle for most of a tile (same parked wait; kept as a separate name for the call sites).
-__device__ __forceinline__ bool tc_mbar_wait_relaxed(uint32_t bar, uint32_t parity) {
-  for (int it = 0; it < tc::WAIT_POLLS; ++it) {
-    uint32_t ok;
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n\t"
-        "selp.u32 %0, 1, 0, p;\n\t}"
-        : "=r"(ok)
-        : "r"(bar), "r"(parity), "r"(tc::WAIT_HINT_NS)
-        : "memory");
-    if (ok) return true;
-  }
-  return false;
-}
-
 __device__ __forceinline__ void tc_ld32(uint32_t taddr, uint32_t (&r)[32]) {
   asm volatile(
       "tcgen05.ld.sync.aligned.32x32b.x32.b32 "
@@ -113,31 +88,6 @@ __device__ __forceinline__ void tc_ld32(uint32_t taddr, uint32_t (&r)[32]) {
         "=r"(r[24]), "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
       : "r"(taddr));
   asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-}
-
-// One poll of two barriers at once, so that the two shared-memory round trips overlap: bit 0 / bit 1 of the result
-// say which phase has completed.
-__device__ __forceinline__ uint32_t tc_try_wait2(uint32_t bar_a, uint32_t par_a, uint32_t bar_b, uint32_t par_b) {
-  uint32_t ok;
-  asm volatile(
-      "{\n\t.reg .pred pa, pb;\n\t.reg .u32 ra, rb;\n\t"
-      "mbarrier.try_wait.parity.shared::cta.b64 pa, [%1], %2, %5;\n\t"
-      "mbarrier.try_wait.parity.shared::cta.b64 pb, [%3], %4, %5;\n\t"
-      "selp.u32 ra, 1, 0, pa;\n\t"
-      "selp.u32 rb, 2, 0, pb;\n\t"
-      "or.b32 %0, ra, rb;\n\t}"
-      : "=r"(ok)
-      : "r"(bar_a), "r"(par_a), "r"(bar_b), "r"(par_b), "r"(tc::WAIT_HINT_NS)
-      : "memory");
-  return ok;
-}
-__device__ __forceinline__ bool tc_wait2(uint32_t bar_a, uint32_t par_a, uint32_t bar_b, uint32_t par_b) {
-  uint32_t done = 0;
-  for (int it = 0; it < tc::WAIT_POLLS; ++it) {
-    done |= tc_try_wait2(bar_a, par_a, bar_b, par_b);
-    if (done == 3) return true;
-  }
-  return false;
 }
 
 }  // namespace uniql

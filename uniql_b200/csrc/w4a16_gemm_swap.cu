@@ -197,7 +197,7 @@ __device__ __forceinline__ SwOut sw_out_of(const SwapParams& p, int T) {
 // One value: bias, SwiGLU product, residual, with the roundings of the separate modules (fp16 result, fp16 SiLU, fp16
 // product, fp16 sum).  Everything optional sits behind a uniform branch: this code runs once per launch, so the
 // instructions it does not fetch are what it saves.
-template <bool PAIR>
+template <bool PAIR, bool RES>
 __device__ __forceinline__ __half sw_value(const SwOut& o, int row, int n, float a, float u) {
   if (o.bias) a += __half2float(o.bias[n]);
   __half h = __float2half_rn(a);
@@ -208,22 +208,23 @@ __device__ __forceinline__ __half sw_value(const SwOut& o, int row, int n, float
     const __half ah = __float2half_rn(gf / (1.0f + expf(-gf)));
     h = __float2half_rn(__half2float(ah) * __half2float(uh));
   }
-  if (o.residual) h = __float2half_rn(__half2float(h) + __half2float(o.residual[(size_t)row * o.ldr + n]));
+  if (RES && o.residual) h = __float2half_rn(__half2float(h) + __half2float(o.residual[(size_t)row * o.ldr + n]));
   return h;
 }
 // Four adjacent columns of one batch row of a plain launch.  c4: column inside the tile.
+template <bool RES>
 __device__ __forceinline__ void sw_finish4(const SwOut& o, int row, int c4, float4 v) {
   const int n = o.n0 + c4;
   if (n >= o.n_out || row >= o.row_end) return;
   __half* d = o.D + (size_t)row * o.ldd + n;
   const float a[4] = {v.x, v.y, v.z, v.w};
-  if (n + 3 < o.n_out && !o.bias && !o.residual && (reinterpret_cast<uintptr_t>(d) & 7u) == 0) {
+  if (n + 3 < o.n_out && !o.bias && !(RES && o.residual) && (reinterpret_cast<uintptr_t>(d) & 7u) == 0) {
     const __half2 lo = __floats2half2_rn(v.x, v.y), hi = __floats2half2_rn(v.z, v.w);
     *reinterpret_cast<uint2*>(d) = make_uint2(*reinterpret_cast<const uint32_t*>(&lo), *reinterpret_cast<const uint32_t*>(&hi));
   } else {
 #pragma unroll
     for (int e = 0; e < 4; ++e)
-      if (n + e < o.n_out) d[e] = sw_value<false>(o, row, n + e, a[e], 0.f);
+      if (n + e < o.n_out) d[e] = sw_value<false, RES>(o, row, n + e, a[e], 0.f);
   }
 }
 
@@ -240,7 +241,7 @@ __device__ __forceinline__ void sw_finish4_tp(const SwOut& o, const CommView& cv
 #pragma unroll
   for (int e = 0; e < 4; ++e) {
     h[e] = __float2half_rn(0.f);
-    if (n + e < o.n_out) d[e] = h[e] = sw_value<PAIR>(o, row, n + e, a[e], b[e]);
+    if (n + e < o.n_out) d[e] = h[e] = sw_value<PAIR, true>(o, row, n + e, a[e], b[e]);
   }
   if (cv.gather_out) tp_feature4(cv, gather_ep, row, n, o.n_out, h);
 }
@@ -260,7 +261,7 @@ __global__ void __launch_bounds__(sw::THREADS, 1)
 w4a16_gemm_swap_kernel(const __grid_constant__ SwapParams p, const __grid_constant__ CUtensorMap xmap,
                        const __grid_constant__ SwapMaps wmaps) {
   using namespace sw;
-  static_assert(GS || !TP, "the exchanges have room for 16 rows");
+  static_assert(GS || (!PAIR && !TP), "above 16 rows: plain outputs only");
   extern __shared__ uint8_t smem_unaligned[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_unaligned) + 1023) & ~(uintptr_t)1023);
   const uint32_t sbase = tc_smem_addr(smem);
@@ -378,8 +379,9 @@ w4a16_gemm_swap_kernel(const __grid_constant__ SwapParams p, const __grid_consta
   // Finishes 16 rows of a tile, held by four warps (one per quarter of the columns; `v`: this lane's column).  A cluster
   // parks them in the activation ring (idle once the last MMA has completed) for the sum over the ranks, below.
   // Otherwise the values of a plain launch are stored straight from the registers (64 bytes per warp and row); a pair
-  // goes through `park` (16 rows of shared memory) and named barrier `bar`, which bring gate and up together.
-  auto emit = [&](const SwOut& o, int c0, const float (&v)[16], uint32_t park, int bar, int gtid) {
+  // (and a tensor-parallel launch) goes through `park`, 16 rows of shared memory, and a barrier of the four epilogue
+  // warps, which bring gate and up together.
+  auto emit = [&](const SwOut& o, int c0, const float (&v)[16], uint32_t park, int gtid) {
     const int col = (warp & 3) * 32 + lane;
     if (p.split > 1) {
 #pragma unroll
@@ -389,17 +391,17 @@ w4a16_gemm_swap_kernel(const __grid_constant__ SwapParams p, const __grid_consta
       tp_epochs(o, gtid, reduce_ep, gather_ep);
 #pragma unroll
       for (int e = 0; e < RC; ++e) tc_sts32(park + e * ROW_BYTES + col * 4, __float_as_uint(v[e]));
-      asm volatile("bar.sync %0, 128;" ::"r"(bar) : "memory");
+      asm volatile("bar.sync 1, 128;" ::: "memory");
       finish_tp(o, 0, min(RC, o.row_end - o.row0), gtid, 128, reduce_ep, gather_ep,
                 [&](int r, int c) { return sw_lds_f4(park + r * ROW_BYTES + c * 4); });
-      asm volatile("bar.sync %0, 128;" ::"r"(bar) : "memory");
+      asm volatile("bar.sync 1, 128;" ::: "memory");
       tp_advance(o, gtid);
     } else if (!PAIR) {
       const int n = o.n0 + col, rows = o.row_end - o.row0 - c0;
       if (n < o.n_out) {
         __half* d = o.D + (size_t)(o.row0 + c0) * o.ldd + n;
         const float bv = o.bias ? __half2float(o.bias[n]) : 0.f;
-        if (o.residual) {
+        if (GS && o.residual) {
           const __half* res = o.residual + (size_t)(o.row0 + c0) * o.ldr + n;
 #pragma unroll
           for (int e = 0; e < RC; ++e)
@@ -414,7 +416,7 @@ w4a16_gemm_swap_kernel(const __grid_constant__ SwapParams p, const __grid_consta
     } else {
 #pragma unroll
       for (int e = 0; e < RC; ++e) tc_sts32(park + e * ROW_BYTES + col * 4, __float_as_uint(v[e]));
-      asm volatile("bar.sync %0, 128;" ::"r"(bar) : "memory");
+      asm volatile("bar.sync 1, 128;" ::: "memory");
       // one value per thread and step: a small loop, because instructions that run once per tile are fetched cold
       const int c = gtid & 63, n = o.n0 + c, rows = min(RC, o.row_end - o.row0 - c0);
       if (n < o.n_out) {
@@ -422,13 +424,13 @@ w4a16_gemm_swap_kernel(const __grid_constant__ SwapParams p, const __grid_consta
         for (int r = gtid >> 6; r < rows; r += 2) {
           const uint32_t a = park + r * ROW_BYTES + c * 4;
           const int row = o.row0 + c0 + r;
-          o.D[(size_t)row * o.ldd + n] = sw_value<true>(o, row, n, sw_lds_f(a), sw_lds_f(a + 256));
+          o.D[(size_t)row * o.ldd + n] = sw_value<true, true>(o, row, n, sw_lds_f(a), sw_lds_f(a + 256));
         }
       }
     }
   };
   // reads the accumulators of 16 rows (both issuers') of tensor-memory tile `acc` and finishes them
-  auto drain = [&](const SwOut& o, uint32_t acc, int c0, uint32_t park, int bar, int gtid) {
+  auto drain = [&](const SwOut& o, uint32_t acc, int c0) {
     uint32_t r0[16], r1[16];
     sw_ld16(acc + c0, r0);
     if (p.nissue == 2) sw_ld16(acc + p.Mb + c0, r1);
@@ -440,7 +442,7 @@ w4a16_gemm_swap_kernel(const __grid_constant__ SwapParams p, const __grid_consta
 #pragma unroll
       for (int e = 0; e < 16; ++e) v[e] += __uint_as_float(r1[e]);
     }
-    emit(o, c0, v, park, bar, gtid);
+    emit(o, c0, v, 0, 0);                        // plain outputs: nothing is parked
   };
 
   if (warp == 0) {
@@ -577,7 +579,7 @@ w4a16_gemm_swap_kernel(const __grid_constant__ SwapParams p, const __grid_consta
               for (int e = 0; e < 16; ++e) acc[e] = fmaf(__uint_as_float(r[e]), cur[j], acc[e]);
             }
         }
-        emit(o, 0, acc, park(), 1, etid);
+        emit(o, 0, acc, park(), etid);
       } else {
         const int buf = p.nbuf == 2 ? (it_tile & 1) : 0;
         const int use = p.nbuf == 2 ? it_tile >> 1 : it_tile;
@@ -585,7 +587,7 @@ w4a16_gemm_swap_kernel(const __grid_constant__ SwapParams p, const __grid_consta
         tc_fence_after();
         const int rows = min(p.Mb, p.M - o.row0);
         for (int c0 = 0; c0 < rows; c0 += RC)
-          drain(o, lane_base + buf * p.nissue * p.Mb, c0, park(), 1, etid);
+          drain(o, lane_base + buf * p.nissue * p.Mb, c0);
         tc_fence_before();
         __syncwarp();
         if (lane == 0) tc_mbar_arrive(bar_tmem_empty + 8 * buf);
@@ -705,13 +707,13 @@ w4a16_gemm_swap_kernel(const __grid_constant__ SwapParams p, const __grid_consta
   if (!GS && p.one_tile && warp >= FIRST_EPI_WARP && tile0 < p.ntiles) {
     // A CTA with a single tile has no next main loop to hide its epilogue behind, and its dequantise warps are idle by
     // now: all twenty warps past the producers drain the accumulator, five groups of four taking 16 rows in turn.
-    const int grp = (warp - FIRST_EPI_WARP) >> 2, gtid = (int)threadIdx.x - FIRST_EPI_WARP * 32 - grp * 128;
+    const int grp = (warp - FIRST_EPI_WARP) >> 2;
     const SwOut o = sw_out_of(p, tile0);
     const int rows = min(p.Mb, p.M - o.row0);
     if (!timed_out && !tc_mbar_wait(bar_tmem_full, 0)) timed_out = true;
     tc_fence_after();
     for (int c0 = grp * RC; c0 < rows; c0 += (FINISH_THREADS / 128) * RC)
-      drain(o, tmem_base + ((uint32_t)((warp & 3) * 32) << 16), c0, xbase + c0 * ROW_BYTES, 1 + grp, gtid);
+      drain(o, tmem_base + ((uint32_t)((warp & 3) * 32) << 16), c0);
   }
   if (p.split > 1) {
     // The parked tile is finished by all twenty warps past the producers (the dequantise warps are idle by now), four
@@ -774,14 +776,14 @@ w4a16_gemm_swap_kernel(const __grid_constant__ SwapParams p, const __grid_consta
             const uint32_t off = (uint32_t)r * ROW_BYTES + c * 4;
             const int row = o.row0 + r;
             const float v = sum_ranks(off);
-            o.D[(size_t)row * o.ldd + n] = sw_value<true>(o, row, n, v, sum_ranks(off + 256));
+            o.D[(size_t)row * o.ldd + n] = sw_value<true, true>(o, row, n, v, sum_ranks(off + 256));
           }
         }
       } else {
 #pragma unroll 1
         for (int idx = ftid; idx < (row1 - row0) * 32; idx += FINISH_THREADS) {
           const int r = row0 + (idx >> 5), c4 = (idx & 31) * 4;
-          sw_finish4(o, o.row0 + r, c4, sum4(r, c4));
+          sw_finish4<GS>(o, o.row0 + r, c4, sum4(r, c4));
         }
       }
     }
@@ -808,7 +810,7 @@ typedef void (*SwapKernel)(const SwapParams, const CUtensorMap, const SwapMaps);
 static SwapKernel swap_kernel(bool gs, bool pair, bool tp) {
   if (tp) return pair ? w4a16_gemm_swap_kernel<true, true, true> : w4a16_gemm_swap_kernel<true, false, true>;
   if (gs) return pair ? w4a16_gemm_swap_kernel<true, true, false> : w4a16_gemm_swap_kernel<true, false, false>;
-  return pair ? w4a16_gemm_swap_kernel<false, true, false> : w4a16_gemm_swap_kernel<false, false, false>;
+  return w4a16_gemm_swap_kernel<false, false, false>;
 }
 
 // Clusters of `split` CTAs that can be resident together (0 if the query fails).
@@ -982,8 +984,9 @@ int launch_gemm_swap(const SwapArgs& a, cudaStream_t stream) {
   p.nproj = a.nproj;
   p.residual = (const __half*)a.residual; p.ldr = a.ldr;
   const bool gs = m <= 16;
+  if (!gs && (a.pair || a.residual || a.comm)) return UNIQL_ESHAPE;   // plain outputs only
   if (a.comm) {
-    if (!gs || (a.comm->reduce && (a.nproj != 1 || a.pair))) return UNIQL_EINVAL;
+    if (a.comm->reduce && (a.nproj != 1 || a.pair)) return UNIQL_EINVAL;
     p.cv = *a.comm;
   }
   {

@@ -202,7 +202,7 @@ w4a16_gemm_tc_kernel(const TcParams p, const __grid_constant__ CUtensorMap amap)
       const int mt = tile % p.mtiles, nt = tile / p.mtiles;
       const int buf = half;
       const uint32_t full_parity = it_tile & 1;
-      if (!timed_out && !tc_mbar_wait_relaxed(bar_tmem_full + 8 * buf, full_parity)) timed_out = true;
+      if (!timed_out && !tc_mbar_wait(bar_tmem_full + 8 * buf, full_parity)) timed_out = true;
       tc_fence_after();
       const int m = (mt * H + half) * BMH + q * 32 + lane;
       const uint32_t taddr = tmem_base + ((uint32_t)(q * 32) << 16) + buf * BN;
@@ -349,8 +349,6 @@ w4a16_gemm_tc_kernel(const TcParams p, const __grid_constant__ CUtensorMap amap)
 bool gemm_tc_supported(int64_t m, int64_t n, int64_t k) {
   return m > 16 && n >= 128 && n % 64 == 0 && k % 128 == 0;
 }
-
-size_t gemm_tc_scratch_bytes(int64_t, int64_t, int64_t) { return 0; }
 
 // Which kernel runs m > 16 rows.  The 256 x 256 tiles of the kernel above reuse activations and weights twice as often as
 // the 128-column tiles of the operand-swapped kernel, whose finer tiles, k-split and shared launches waste less of the

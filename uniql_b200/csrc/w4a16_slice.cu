@@ -10,7 +10,7 @@
 //     through the 64-column scale permutation.
 //   * w4a16_dequantize_rows_kernel: fp16 (q - 8) * s of chosen input rows, written in the nn.Linear layout
 //     [column][kept row] that uniql_w4a16_quantize reads (o_proj / out_proj slicing re-quantises, :632-650).
-// Both are gathers of 4-byte words: memory-bound, run once per layer at load time.
+// Memory-bound gathers (4-byte words of the columns, 16-byte pieces of the rows), run once per layer at load time.
 #include "common.cuh"
 
 namespace uniql {
