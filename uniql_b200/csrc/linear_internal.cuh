@@ -61,6 +61,11 @@ struct DecodeArgs {
 
 // CTA-tiled decode kernel (w4a16_gemv.cu): single-GPU launches, activations already transformed.
 size_t gemv_scratch_bytes(int64_t m, int64_t k, const int64_t* n, int nproj, int epilogue);
+// Grid of such a launch: CTAs, those of them that share a column group (k-split), CTAs that are resident at a time.
+struct GemvGrid {
+  int ctas, split, slots;
+};
+GemvGrid gemv_grid(int64_t m, int64_t k, const int64_t* n, int nproj, int epilogue);
 int launch_gemv_group(const DecodeArgs& a, const __half* A, int64_t lda, bool early_weights, cudaStream_t stream);
 
 // m <= 16.  Scratch bytes the launch needs (tickets included).
@@ -99,6 +104,12 @@ struct SwapArgs {
 };
 bool gemm_swap_supported(int64_t m, int64_t k, const int64_t* n, int nproj);
 int launch_gemm_swap(const SwapArgs& a, cudaStream_t stream);
+// Work split of such a launch with `ctiles` column tiles (128 columns, or 64 + 64 of a pair): waves of tiles, CTAs that share
+// a tile, k-blocks of the busiest CTA per tile.  waves = 0: the kernel cannot be launched.
+struct SwapGrid {
+  int waves, split, kblocks;
+};
+SwapGrid gemm_swap_grid(int64_t m, int64_t k, int ctiles);
 double gemm_swap_cycles(int64_t m, int64_t k, int ctiles);   // modelled SM cycles of such a launch
 
 // Hadamard transform of fp16 rows (used by the fused linear); signals dependents early when pdl is set.

@@ -1083,7 +1083,31 @@ static int launch_variant(const DecodeParams& p, const DecodePlan& pl, bool pdl,
   return UNIQL_OK;
 }
 
+// Which kernel runs 5 to 16 rows.  The tensor-core kernel's work per weight does not grow with the rows, while the tiled
+// kernel stages rows x k activations in every CTA: 14336 x 4096 in us, tiled / tensor core, 4 rows 9.8 / 11.4, 5 rows
+// 13.1 / 12.5, 8 rows 13.7 / 12.6, 16 rows 19.5 / 12.7; 1024 x 4096 at 5 rows 5.8 / 5.2.  Up to 8 rows (one batch tile of
+// the tiled kernel) two kinds of launch stay on the tiled kernel, if no more than four of its CTAs share a column group:
+//   * the tensor-core kernel needs a second wave of tiles, and the tiled one fills 5/6 of the resident CTAs or more in a
+//     single wave: gate + up of 18944 x 3584 21.0 / 22.3, 32000 x 3584 19.8 / 20.4, 37888 x 2048 13.2 / 14.7; with a
+//     smaller filling not: gate + up of 12160 x 4096 21.6 / 20.5 (192 of 296);
+//   * four CTAs or more of the tensor-core kernel share a tile and have eight k-blocks or fewer each, so that the cluster
+//     sum is a large part, and the tiled kernel has a CTA for nearly every SM: 4096 x 4096 7.2 / 7.6, 3328 x 3072
+//     6.6 / 7.6; but 4096 x 8192 10.7 / 10.2, and gate + up of 2048 x 2048 (128 CTAs) 6.7 / 6.4.
+// The rule knows nothing of a communicator: a step of a tensor-parallel layer has the sums of the plain launch.
 constexpr int kSwapMinRows = 5;
+static bool swap_kernel_runs(const DecodeArgs& a, const int64_t* n) {
+  if (a.m < kSwapMinRows || !gemm_swap_supported(a.m, a.k, n, a.nproj)) return false;
+  if (a.m > 8) return true;
+  const GemvGrid t = gemv_grid(a.m, a.k, n, a.nproj, a.epilogue);
+  if (t.split > 4 || t.ctas > t.slots) return true;
+  int ctiles = 0;
+  if (a.epilogue == UNIQL_EPILOGUE_SWIGLU) ctiles = (int)(n[0] / 64);
+  else for (int i = 0; i < a.nproj; ++i) ctiles += (int)((n[i] + 127) / 128);
+  const SwapGrid s = gemm_swap_grid(a.m, a.k, ctiles);
+  if (s.waves == 2) return 6 * t.ctas < 5 * t.slots;
+  if (s.split >= 4 && s.kblocks <= 8) return 16 * t.ctas < 15 * device_info().sm_count;
+  return s.waves > 0;
+}
 
 // What the exchange areas of a communicator have room for.
 static int comm_fits(const DecodeArgs& a) {
@@ -1133,12 +1157,7 @@ int launch_decode(const DecodeArgs& a, cudaStream_t stream) {
     }
     // the transform is a launch of its own that starts when everything in front of it has ended
     const bool early_weights = a.early_weights || a.hadamard_dim != 0;
-    // From five rows on, with and without a communicator (a step of a tensor-parallel layer has the sums of the plain
-    // launch), the tensor-core kernel with exact codes as the operand and fp32 group scales (the arithmetic of the
-    // tiled kernel) is faster: its work per weight does not grow with the rows, while the tiled kernel stages rows x k
-    // activations in every CTA.  14336 x 4096 in us, tiled / tensor core: 4 rows 9.8 / 11.4, 8 rows 12.8 / 11.7, 16 rows
-    // 18.6 / 11.7; 4096 x 14336: 11.8 / 12.6, 13.9 / 12.7, 18.7 / 12.8; 4096 x 4096: 6.7 / 7.6, 7.1 / 7.5, 8.5 / 7.6.
-    if (a.m >= kSwapMinRows && gemm_swap_supported(a.m, a.k, n, a.nproj)) {
+    if (swap_kernel_runs(a, n)) {
       LinearArgs la[kMaxProj];
       void* ds[kMaxProj];
       for (int i = 0; i < a.nproj; ++i) {

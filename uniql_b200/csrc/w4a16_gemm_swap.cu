@@ -933,6 +933,15 @@ double gemm_swap_cycles(int64_t m, int64_t k, int ctiles) {
   return swap_shape(m, k, ctiles, m <= 16, swap_forced_split()).cycles;
 }
 
+SwapGrid gemm_swap_grid(int64_t m, int64_t k, int ctiles) {
+  const bool gs = m <= 16;
+  if (swap_set_attributes(gs, false, false) != UNIQL_OK) return SwapGrid{0, 0, 0};
+  const SwapShape s = swap_shape(m, k, ctiles, gs, swap_forced_split());
+  if (s.split < 1) return SwapGrid{0, 0, 0};
+  const int sms = device_info().sm_count, groups = (int)(k / 128);
+  return SwapGrid{s.split > 1 ? 1 : (ctiles * s.rtiles + sms - 1) / sms, s.split, (groups + s.split - 1) / s.split};
+}
+
 bool gemm_swap_supported(int64_t m, int64_t k, const int64_t* n, int nproj) {
   if (m < 1 || k % 128 || nproj < 1 || nproj > kMaxProj) return false;
   for (int i = 0; i < nproj; ++i)

@@ -810,6 +810,13 @@ size_t gemv_scratch_bytes(int64_t m, int64_t k, const int64_t* n, int nproj, int
   return UNIQL_SCRATCH_COUNTER_BYTES + (plan.partial_bytes + 255) / 256 * 256;
 }
 
+GemvGrid gemv_grid(int64_t m, int64_t k, const int64_t* n, int nproj, int epilogue) {
+  const int64_t nv = virtual_width(n, nproj);
+  const GemvPlan plan = plan_gemv(m, nv, k, epilogue == UNIQL_EPILOGUE_SWIGLU);
+  return GemvGrid{(int)((nv / 64 + plan.WN - 1) / plan.WN) * plan.S, plan.S,
+                  device_info().sm_count * (plan.MT == 1 ? kCtasMt1 : 2)};
+}
+
 // A: the activations the kernel multiplies with (already transformed if the layer has an online Hadamard).
 int launch_gemv_group(const DecodeArgs& a, const __half* A, int64_t lda, bool early_weights, cudaStream_t stream) {
   if (a.nproj < 1 || a.nproj > kMaxProj || a.m < 1 || a.m > 16 || a.k % 128) return UNIQL_ESHAPE;
