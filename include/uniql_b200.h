@@ -255,10 +255,10 @@ int uniql_w4a16_linear_allreduce(void* comm, const void* A, int64_t lda, const v
  *     launch the linear's weight stream overlaps (in the slot-balanced kernel's own prologue for m <= 4).
  * Each projection is described by plain pointers and sizes (see uniql_w4a16_linear for B, s, bias, D, n, n_out).
  * scratch: at least uniql_w4a16_group_scratch_bytes(...) bytes, 256-byte aligned, first UNIQL_SCRATCH_COUNTER_BYTES
- * zero before the first call (every call leaves them zero).  The launch starts fetching weights and scales before the
- * kernel in front of it has ended: between a kernel that writes them and this call the stream must hold something other
- * than grouped launches and uniql_silu_mul (any other kernel, a call of uniql_w4a16_linear, or a synchronisation).  Activations, bias,
- * residual and outputs have no such restriction, and uniql_w4a16_linear and the other single-projection calls have none.
+ * zero before the first call (every call leaves them zero).  The weights and scales must not be written by the kernel
+ * that immediately precedes this call in the stream (the launch starts fetching them before that kernel has ended);
+ * activations, bias, residual and outputs have no such restriction, and uniql_w4a16_linear and the other single-projection
+ * calls have none.
  */
 #define UNIQL_MAX_PROJ 4
 enum { UNIQL_EPILOGUE_NONE = 0, UNIQL_EPILOGUE_SWIGLU = 1 };

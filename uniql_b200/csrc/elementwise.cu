@@ -10,8 +10,8 @@ __global__ void __launch_bounds__(256) silu_mul_kernel(const __half* __restrict_
                                                       const __half* __restrict__ up, int64_t ldu,
                                                       __half* __restrict__ out, int64_t ldo, int64_t rows,
                                                       int64_t cols8) {
-  pdl_launch_dependents();
   pdl_wait();                                   // gate and up come from the launch right before this one
+  pdl_launch_dependents();                      // behind the wait: what starts early may rely on what stands in front
   const int64_t total = rows * cols8;
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (int64_t)gridDim.x * blockDim.x) {
     const int64_t r = i / cols8, c = (i - r * cols8) * 8;

@@ -32,8 +32,8 @@
 // four rows the online Hadamard transform of the activations runs in the kernel's own prologue.
 //
 // Where the predecessor cannot have written the weights, a launch carries the programmatic-dependent-launch attribute, fills
-// its rings, releases its own dependents and only then waits for its predecessor.  Measured against the tiled kernel this kernel is slower (its reduction crosses global
-// memory); it is kept as a tested alternative.
+// its rings, waits for its predecessor and releases its own dependents.  Measured against the tiled kernel this kernel is
+// slower (its reduction crosses global memory); it is kept as a tested alternative.
 //
 // Roofline: HBM.  Algorithmic bytes per launch = sum over projections of k*n/2 + (k/128)*n*2 + m*n_out*2, + m*k*2.
 #include "common.cuh"
@@ -688,8 +688,8 @@ __global__ void __launch_bounds__(WARPS * 32, MINB) w4a16_decode_kernel(const __
   }
   // Let the next kernel in the stream start its own weight prefetch, then wait for the producer of the activations.
   STAMP(1);
-  pdl_launch_dependents();
   pdl_wait();
+  pdl_launch_dependents();
   STAMP(2);
 
   bool timed_out = false;

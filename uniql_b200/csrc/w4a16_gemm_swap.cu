@@ -286,9 +286,6 @@ w4a16_gemm_swap_kernel(const __grid_constant__ SwapParams p, const __grid_consta
   const int total_it = my_tiles * KB;
   const int tmem_w0 = TMEM_COLS - p.nst * (BK / 2);   // weight tile of stage s: columns tmem_w0 + 64 s
 
-  // the next kernel in the stream may start its own set-up and weights; where this launch waits for its predecessor first,
-  // behind that wait, so that what starts behind this launch may rely on the predecessor too
-  if (p.early_weights) pdl_launch_dependents();
   // Packed words of k-block kb of column tile (pi, lt): two boxes, one barrier.
   auto load_packed = [&](int pi, int lt, int kb, int sp) {
     const int x0 = PAIR ? lt * 128 : lt * 256;
@@ -337,10 +334,7 @@ w4a16_gemm_swap_kernel(const __grid_constant__ SwapParams p, const __grid_consta
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
   bool timed_out = false;
-  if (!p.early_weights) {
-    pdl_wait();                                  // before the first scale is read
-    pdl_launch_dependents();
-  }
+  if (!p.early_weights) pdl_wait();              // before the first scale is read
 
   // TP: finishes rows [r0, r1) of a tile with `nthreads` threads, four columns of a row per thread and step; `quad` delivers
   // the sums of four adjacent columns of the tile.  kQuads divides every nthreads, so a thread stays in one 64-column block.
@@ -473,7 +467,10 @@ w4a16_gemm_swap_kernel(const __grid_constant__ SwapParams p, const __grid_consta
       // Programmatic dependent launch: everything up to here (barriers, tensor memory, the first weight tiles and their
       // conversion) ran while the producer of the activations was still finishing; the activation tiles are the only
       // thing that has to wait for it.  Results (and the residual) are touched after MMAs that consumed those tiles.
+      // The next kernel in the stream may start its own set-up and weights from here on: behind the wait, so that it may
+      // rely on everything in front of this launch having ended.
       pdl_wait();
+      pdl_launch_dependents();
       int s = 0;
       uint32_t ph = 0;
       for (int T = tile0; T < p.ntiles && !timed_out; T += tile_step) {

@@ -21,7 +21,7 @@
 // distributed shared memory, for S > 8 they write fp32 partials to scratch and the last one to arrive (atomic ticket,
 // no spinning) adds them in a fixed order -> deterministic results, no inter-CTA waits outside a cluster barrier.
 // Every launch is a programmatic dependent: where the caller rules out that the preceding kernel wrote the weights it starts
-// its weight stream, releases its own dependents and only then waits for the producer of its activations.
+// its weight stream, then waits for the producer of its activations and releases its own dependents.
 //
 // Grouped launches.  Up to four projections that read the same activations form one launch: their 64-column blocks
 // are laid side by side in one virtual column space (block by block for q/k/v; gate and up blocks interleaved for a
@@ -251,7 +251,7 @@ w4a16_gemv_kernel(const __grid_constant__ GemvParams p) {
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
   }
   __syncwarp();
-  if (!p.early_weights) pdl_wait();    // ahead of the release below: what starts behind this launch may rely on it
+  if (!p.early_weights) pdl_wait();
   // ---- start streaming weights before anything else: one TMA tile per group and 64-column block ----
   if (has_work && lane == 0) {
     for (int s = 0; s < p.R; ++s)
@@ -260,9 +260,10 @@ w4a16_gemv_kernel(const __grid_constant__ GemvParams p) {
         tma_load_slot(ring_base + s * kSlotBytes, wmap, lb * 128, 8 * (g0 + s), bar0 + s * 8, pol);
       }
   }
-  // Let the next kernel in the stream start its own weight prefetch, then wait for the producer of A.
-  pdl_launch_dependents();
+  // Wait for the producer of A, then let the next kernel in the stream start its own weight prefetch.  In this order a kernel
+  // that starts behind this launch may rely on everything in front of it having ended; the other one was no faster.
   pdl_wait();
+  pdl_launch_dependents();
   if ((p.cv.reduce || p.cv.gather_out) && tid < p.WN) {
     // one per 64-column block (per gate/up pair); read behind the wait: the preceding launch may have advanced them
     const int vb = blockIdx.x * p.WN + tid;

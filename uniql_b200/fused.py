@@ -7,10 +7,9 @@ moves, so for up to 16 rows the functions below issue one grouped kernel (uniql_
 to 128 rows the projections still share one launch (plain outputs, the elementwise maths in PyTorch); larger batches
 run the same modules one after the other on the tensor-core kernels, exactly as the reference does it.  All take and return the tensors the reference's code would.
 
-The grouped launches start fetching packed weights and scales before the kernel in front of them has ended.  So a program
-that writes a layer's buffers on the GPU and calls one of these functions on the layer right behind, with nothing but
-other grouped launches in between on the stream, has to put a synchronisation (or any other kernel) there; the modules'
-own forward has no such rule.
+The grouped launches start fetching packed weights and scales before the kernel in front of them has ended, so that kernel
+must not be the one that writes them: a program that changes a layer's buffers on the GPU and calls one of these functions
+on the layer right behind puts another kernel or a synchronisation in between.  The modules' own forward has no such rule.
 """
 from __future__ import annotations
 
