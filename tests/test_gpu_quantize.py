@@ -164,3 +164,48 @@ def test_a_layer_runs_right_behind_the_kernel_that_packs_it(rows):
         got = [W4A16B16O16Linear.from_fp16(lin)(x) for lin in srcs]
         for g, w in zip(got, want):
             assert torch.equal(g, w)
+
+
+@pytest.mark.parametrize("rows", [1, 8, 64])
+def test_captured_chain_reads_what_the_graph_packs(rows):
+    """In a capture a linear right behind another linear starts its weights early, one behind the packing kernel may not: a
+    graph that packs a layer and runs it between two other linears gives, on every replay, the result of the weight of that
+    replay."""
+    from uniql_b200 import ops
+    from uniql_b200.quantize.quant_linear_layers import W4A16B16O16Linear
+    n, k = 4096, 4096                 # large enough for the early start
+    x = make_acts(rows, rows, k).cuda()
+    fixed = W4A16B16O16Linear.from_fp16(torch.nn.Linear(k, n, bias=False, device="cuda", dtype=torch.float16))
+    src = torch.empty(n, k, dtype=torch.float16, device="cuda")
+    spare = torch.empty(1, n, dtype=torch.float16, device="cuda")
+    weights = [(torch.randn(n, k, generator=torch.Generator().manual_seed(i)) * 0.02).half().cuda() for i in range(3)]
+
+    def step():
+        a = fixed(fixed(x))
+        _, packed, scales = ops.w4a16_quantize(src, n_pad=n, want_ref=False)
+        ops.w4a16_linear_group(x[:0], [(fixed.weight, fixed.scale, None, n)], outs=[spare])      # no rows: launches nothing
+        b = ops.w4a16_linear(a, packed, scales, None, n)
+        return a, b, fixed(b)
+
+    want = []
+    for w in weights:
+        src.copy_(w)
+        torch.cuda.synchronize()
+        _, packed, scales = ops.w4a16_quantize(src, n_pad=n, want_ref=False)
+        torch.cuda.synchronize()
+        a = fixed(fixed(x))
+        b = ops.w4a16_linear(a, packed, scales, None, n)
+        want.append((a, b, fixed(b)))
+    stream = torch.cuda.Stream()
+    with torch.cuda.stream(stream):
+        step()
+        torch.cuda.synchronize()
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph, stream=stream):
+            got = step()
+        for _ in range(3):
+            for w, ref in zip(weights, want):
+                src.copy_(w)
+                graph.replay()
+                torch.cuda.synchronize()
+                assert all(torch.equal(g, r) for g, r in zip(got, ref))

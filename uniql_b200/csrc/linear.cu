@@ -25,6 +25,40 @@ const DeviceInfo& device_info() {
   return info[dev];
 }
 
+// What stands in front of a launch is known while its stream is captured: if the only thing the next node will depend on is
+// the last linear that this thread captured, no other kernel can have written the weights in between (and that launch
+// releases its dependents behind its own wait, so everything in front of it has ended).  A decode step replayed from a
+// graph then keeps the early weight stream between linears called one by one; outside a capture the calls wait.
+// Capture ids are unique in the process, so a mark of another capture never matches.
+struct CaptureTail {
+  bool active;                 // the stream is being captured ...
+  unsigned long long id;
+  cudaGraphNode_t node;        // ... and the next node will depend on this one alone (nullptr: on several, or on none)
+};
+static CaptureTail capture_tail(cudaStream_t stream) {
+  CaptureTail t{false, 0, nullptr};
+  cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+  const cudaGraphNode_t* deps = nullptr;
+  const cudaGraphEdgeData* edges = nullptr;
+  size_t ndeps = 0;
+  if (cudaStreamGetCaptureInfo_v3(stream, &status, &t.id, nullptr, &deps, &edges, &ndeps) != cudaSuccess) {
+    (void)cudaGetLastError();
+    return t;
+  }
+  t.active = status == cudaStreamCaptureStatusActive;
+  if (t.active && ndeps == 1) t.node = deps[0];
+  return t;
+}
+static thread_local CaptureTail g_last_linear{false, 0, nullptr};
+static bool behind_own_linear(const CaptureTail& t) {
+  return t.node && t.id == g_last_linear.id && t.node == g_last_linear.node;
+}
+// Called right behind every linear that has been launched (m > 0) and may be part of a capture.
+static int note_linear(int launch_status, cudaStream_t stream) {
+  if (launch_status == UNIQL_OK) g_last_linear = capture_tail(stream);
+  return launch_status;
+}
+
 static inline size_t align_up(size_t v, size_t a) { return (v + a - 1) / a * a; }
 
 static bool use_tc(int64_t m, int64_t n, int64_t k) { return m > 16 && gemm_tc_supported(m, n, k); }
@@ -182,9 +216,14 @@ extern "C" int uniql_w4a16_linear(const void* A, int64_t lda, const void* B, con
 
   uniql_w4a16_proj q;
   q.B = B; q.s = s; q.bias = bias; q.D = D; q.ldd = ldd; q.n = n; q.n_out = n_out;
+  // the query costs ~0.2 us of host time per call; below 4 MB of packed weights an early start gains nothing to speak of
+  // (1024 x 4096 at one row 7.3 us with and without, 14336 x 4096 9.0 / 10.1)
+  const CaptureTail tail = n * k >= (int64_t)1 << 23 ? capture_tail(stream) : CaptureTail{false, 0, nullptr};
+  const bool early = behind_own_linear(tail);
+  auto done = [&](int st) { return tail.active ? note_linear(st, stream) : st; };
   if (m <= 16)
-    return group_launch(nullptr, false, 0, A, lda, m, k, &q, 1, UNIQL_EPILOGUE_NONE, nullptr, 0, hadamard_dim, nullptr, 0,
-                        scratch, scratch_bytes, status_word, stream);
+    return done(group_launch(nullptr, early, 0, A, lda, m, k, &q, 1, UNIQL_EPILOGUE_NONE, nullptr, 0, hadamard_dim, nullptr, 0,
+                             scratch, scratch_bytes, status_word, stream));
 
   // m > 16: Hadamard (if any) as its own kernel into scratch, then the tensor-core kernels
   const __half* Ain = (const __half*)A;
@@ -203,7 +242,7 @@ extern "C" int uniql_w4a16_linear(const void* A, int64_t lda, const void* B, con
   if (tc) {
     LinearArgs a;
     a.B = B; a.s = s; a.bias = bias; a.ldd = ldd; a.n = n; a.n_out = n_out; a.k = k; a.status_word = status_word;
-    return launch_gemm_tc(a, Ain, lda, (__half*)D, m, hadamard_dim != 0, stream);
+    return done(launch_gemm_tc(a, Ain, lda, (__half*)D, m, early || hadamard_dim != 0, stream));
   }
   const size_t slab_bytes = scratch_bytes - (hadamard_dim ? align_up((size_t)m * k * 2, 256) : 0);
   for (int64_t m0 = 0; m0 < m; m0 += 16) {
@@ -220,8 +259,9 @@ extern "C" int uniql_w4a16_linear_group(const void* A, int64_t lda, int64_t m, i
                                         const uniql_w4a16_proj* proj, int nproj, int epilogue, const void* residual,
                                         int64_t ldr, int64_t hadamard_dim, const uniql_prefetch* next, int nnext,
                                         void* scratch, size_t scratch_bytes, int* status_word, void* stream) {
-  return uniql::group_launch(nullptr, true, 0, A, lda, m, k, proj, nproj, epilogue, residual, ldr, hadamard_dim, next, nnext,
-                             scratch, scratch_bytes, status_word, (cudaStream_t)stream);
+  const int st = uniql::group_launch(nullptr, true, 0, A, lda, m, k, proj, nproj, epilogue, residual, ldr, hadamard_dim, next,
+                                     nnext, scratch, scratch_bytes, status_word, (cudaStream_t)stream);
+  return m > 0 ? uniql::note_linear(st, (cudaStream_t)stream) : st;   // without rows nothing is launched
 }
 
 static int group_tp(void* comm, int flags, bool early_weights, int64_t col_offset, int64_t k_offset, const void* A, int64_t lda,
