@@ -108,8 +108,8 @@ static int group_launch(const CommView* cv, bool early_weights, int64_t k_offset
         ++npf;
       }
   if (m > 16) {
-    // 17..128 rows: the projections share one launch of the operand-swapped tensor-core kernel (plain outputs only:
-    // the elementwise epilogues, the transform and the tensor-parallel exchanges belong to the decode kernel)
+    // 17..128 rows: the projections share one launch of the operand-swapped tensor-core kernel (plain outputs only: the
+    // elementwise epilogues, the transform and the tensor-parallel exchanges end at 16 rows)
     if (m > 128 || cv || epilogue != UNIQL_EPILOGUE_NONE || residual || hadamard_dim) return UNIQL_ESHAPE;
     if (lda < k || lda % 8 != 0 || !A || !aligned16(A)) return UNIQL_EINVAL;
     LinearArgs la[UNIQL_MAX_PROJ];

@@ -59,7 +59,7 @@ struct DecodeArgs {
   size_t prefetch_bytes[4];
 };
 
-// CTA-tiled decode kernel (w4a16_gemv.cu): single-GPU launches, activations already transformed.
+// CTA-tiled decode kernel (w4a16_gemv.cu); activations already transformed.
 size_t gemv_scratch_bytes(int64_t m, int64_t k, const int64_t* n, int nproj, int epilogue);
 // Grid of such a launch: CTAs, those of them that share a column group (k-split), CTAs that are resident at a time.
 struct GemvGrid {

@@ -37,7 +37,9 @@
 // with another k may run), so the lowest unfinished tile never waits for a higher one; waits are bounded.
 //
 // Bound: weight stream (HBM) below ~128 rows, tensor pipe above; in practice the per-stage chain of the dequantise warps
-// (~260 issued instructions per warp and stage) and the fixed cost of a launch.
+// (13 instructions per packed word, 9 with GS, and ~110 per warp and stage: ~320 or ~250) and the fixed cost of a launch.
+// All 24 warps together issue 1961 warp instructions per stage at 64 rows, 1631 at 16 (14336 x 4096, counters); the SMs that
+// work issue on 84 % and 79 % of their cycles.
 // Every mbarrier wait is bounded; a wait that gives up sets UNIQL_STATUS_WAIT_TIMEOUT and the kernel drains.
 #include "common.cuh"
 #include "linear_internal.cuh"

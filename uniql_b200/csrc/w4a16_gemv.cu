@@ -1,4 +1,5 @@
-// Decode-regime W4A16 linear (m <= 16; launch_decode uses it up to 4 rows) for sm_100a: a weight-streaming skinny GEMM.
+// Decode-regime W4A16 linear (m <= 16; launch_decode uses it up to 4 rows, and up to 8 where it is the
+// faster one) for sm_100a: a weight-streaming skinny GEMM.
 //
 // Replaces the small-batch instantiations of UniQL's Marlin kernel
 // (csrc/linear/marlin_gemm_kernel.cuh:176-740, tile table :792-800) while consuming the very same

@@ -5,7 +5,8 @@ The reference's blocks call their quantized linears one by one and glue them wit
 (:104-106), `residual + o_proj(...)`.  At decode sizes every one of those launches costs more than the bytes it
 moves, so for up to 16 rows the functions below issue one grouped kernel (uniql_w4a16_linear_group) per step; up
 to 128 rows the projections still share one launch (plain outputs, the elementwise maths in PyTorch); larger batches
-run the same modules one after the other on the tensor-core kernels, exactly as the reference does it.  All take and return the tensors the reference's code would.
+run the same modules one after the other on the tensor-core kernels, exactly as the reference does it.  All take and
+return the tensors the reference's code would.
 
 The grouped launches start fetching packed weights and scales before the kernel in front of them has ended, so that kernel
 must not be the one that writes them: a program that changes a layer's buffers on the GPU and calls one of these functions
@@ -18,8 +19,8 @@ import torch.nn.functional as F
 
 from . import ops
 
-DECODE_ROWS = 16         # the decode kernel: SwiGLU, residual and Hadamard inside the launch
-GROUP_ROWS = 128         # plain outputs of several projections in one launch (tensor-core kernel above 16 rows)
+DECODE_ROWS = 16         # SwiGLU, residual and Hadamard inside the launch
+GROUP_ROWS = 128         # plain outputs of several projections in one launch
 
 
 def _layer(mod):
